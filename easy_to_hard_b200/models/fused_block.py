@@ -140,8 +140,9 @@ def _row_parallel_fused(x_in: torch.Tensor, w: torch.Tensor, residual: torch.Ten
 def block_forward(x: torch.Tensor, w: Dict[str, torch.Tensor], freqs: torch.Tensor,
                   pos: torch.Tensor, shape: BlockShape, keep: bool = False):
     """x [T, dim] (T = B*S, or B*S/tp rows under sequence parallelism). ``w`` holds bf16
-    ``wqkv, wo, w1, w3, w2`` and the two norm weights. Returns ``out`` and, with ``keep``, the
-    intermediates the backward needs."""
+    ``wqkv, wo, w1, w3, w2`` and the two norm weights; ``pos`` the positions of the B*S tokens, those
+    of a sequence consecutive and every sequence from the same one on. Returns ``out`` and, with
+    ``keep``, the intermediates the backward needs."""
     H, Hkv, D = shape.n_head, shape.n_kv, shape.head_dim
     sp = shape.sequence_parallel and shape.tp > 1
     fused_sp = sp and p2p_reduce_enabled()
@@ -156,8 +157,10 @@ def block_forward(x: torch.Tensor, w: Dict[str, torch.Tensor], freqs: torch.Tens
         xn1 = Fn.rmsnorm(x, w["attention_norm"], shape.eps)
         xn1f = _sp_gather(xn1, shape) if sp else xn1
     T = xn1f.shape[0]
-    qkv = gemm.linear(xn1f, w["wqkv"])
-    Fn.rope(qkv, freqs, pos, H + Hkv, D, out=qkv)          # q and k heads, in place
+    # q and k heads rotated in the epilogue; the rows are whole sequences from position pos[0] on
+    qkv = gemm.linear_qkv_rope(xn1f, w["wqkv"], torch.empty(
+        T, (H + 2 * Hkv) * D, dtype=xn1f.dtype, device=xn1f.device), freqs=freqs, pos_base=pos,
+        sq=shape.S, n_head=H, n_kv=Hkv, head_dim=D)
     q = qkv[:, : H * D].view(shape.B, shape.S, H, D)
     k = qkv[:, H * D: (H + Hkv) * D].view(shape.B, shape.S, Hkv, D)
     v = qkv[:, (H + Hkv) * D:].view(shape.B, shape.S, Hkv, D)
@@ -183,8 +186,11 @@ def block_forward(x: torch.Tensor, w: Dict[str, torch.Tensor], freqs: torch.Tens
         xn2 = Fn.rmsnorm(h, w["ffn_norm"], shape.eps)
     if xn2f is None:
         xn2f = _sp_gather(xn2, shape) if sp else xn2
-    g, u = gemm.linear_dual(xn2f, w["w1"], w["w3"])
-    act = Fn.swiglu(g, u)
+    if keep:                       # the backward needs both products
+        g, u = gemm.linear_dual(xn2f, w["w1"], w["w3"])
+        act = Fn.swiglu(g, u)
+    else:
+        act = gemm.linear_swiglu(xn2f, w["w1"], w["w3"])
     if shape.tp == 1:
         out = gemm.linear_residual(act, w["w2"], h)
     elif fused_sp:

@@ -259,7 +259,7 @@ __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0,
         float y = x;
         if (!is_v) y = (d & 1) ? (x * cj[j] + partner * sj[j]) : (x * cj[j] - partner * sj[j]);
         const __nv_bfloat16 yb = __float2bfloat16_rn(y);
-        if (is_q) {
+        if (is_q || p.kcache == nullptr) {
           static_cast<__nv_bfloat16*>(p.out)[(long long)t * p.ldo + f] = yb;
         } else if (posj[j] < p.smax) {
           cache[(((long long)bj[j] * p.n_kv + hk) * p.smax + posj[j]) * D + d] = yb;
@@ -322,6 +322,24 @@ __device__ __forceinline__ RopePre rope_prepare(const E2hGemmParams& p, int f) {
     r.sj = __bfloat162float(cs.y);
   }
   return r;
+}
+
+// (cos, sin) of feature f (rope_prepare's `r`) for N consecutive tokens of whole sequences; (1, 0)
+// where there is nothing to rotate.
+template <int N>
+__device__ __forceinline__ void rope_factors(const E2hGemmParams& p, const RopePre& r, int f, int t0,
+                                             int t_end, __nv_bfloat162* cs) {
+  const __nv_bfloat162* tab = static_cast<const __nv_bfloat162*>(p.freqs) + (r.d >> 1);
+  const int half = p.head_dim / 2;
+  const bool turns = !r.is_v && f < p.F;
+  int s = t0 % p.sq;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int pos = r.pos0 + s;
+    if (++s == p.sq) s = 0;
+    cs[j] = (turns && t0 + j < t_end && pos < p.smax) ? tab[(long long)pos * half]
+                                                      : __floats2bfloat162_rn(1.f, 0.f);
+  }
 }
 
 // Final bf16 value of 8 consecutive tokens of one feature into the shared tile:
@@ -437,7 +455,7 @@ __device__ __forceinline__ void flush_tile(const E2hGemmParams& p, const __nv_bf
       const int D = p.head_dim;
       const int head = f / D;
       const int d = f - head * D;
-      if (head >= p.n_head) {
+      if (head >= p.n_head && p.kcache != nullptr) {
         const bool is_k = head < p.n_head + p.n_kv;
         const int hk = is_k ? head - p.n_head : head - p.n_head - p.n_kv;
         const int b = t / p.sq;

@@ -10,8 +10,15 @@
 //     feature each) write 32-token chunks into a [token][feature] staging buffer and one thread
 //     issues cp.async.bulk.tensor stores of full 256-byte rows; a residual operand comes in the
 //     same way (TMA load of the matching chunk) instead of 2-byte strided loads.
-// Epilogues without a staged form (fp32 outputs, RoPE + KV scatter, weight-gradient
-// accumulation) use the per-thread path of gemm_epilogue.cuh and still get the overlap.
+//   * the RoPE + KV-cache epilogue rotates in registers (the partner of a pair sits in the next
+//     lane, the 32 (cos, sin) pairs of a chunk are fetched while the accumulator is read) and leaves
+//     through the same staging buffer as 16-byte stores to the query rows and the cache rows. One
+//     feature per thread and 2-byte stores one cache row apart held the whole prompt GEMM to a quarter
+//     of its rate: 22432 x 10240 x 8192, 6.47 -> 2.62 ms (plain stores
+//     2.51);
+//   * a gate / up product with SwiGLU is one CTA-pair tile as wide as any other (see SWI below).
+// Epilogues without a staged form (fp32 outputs, weight-gradient accumulation) use the per-thread
+// path of gemm_epilogue.cuh and still get the overlap.
 // Every wait is bounded; on a time-out the roles stop, the status word is set and the CTA
 // still reaches its final barrier and frees its tensor memory.
 #include <cuda.h>
@@ -118,13 +125,57 @@ __device__ __forceinline__ PTile tile_at(const E2hGemmParams& p, const PCtrl* ct
   return t;
 }
 
+// Destination of one 8-feature vector of a staged [32 tokens][128 features] chunk of the RoPE + KV
+// epilogue: thread `et` of the 128 always moves the same features, rows et / 16 + 8 u, so the
+// divisions by the head size and the sequence length are per tile and per chunk.
+struct RopeRows {
+  __nv_bfloat16* base;      // row 0 of the queries, or of the keys / values of this head
+  int f, is_q, pos0;
+  __device__ __forceinline__ void prepare(const E2hGemmParams& p, int pos0_, int f_) {
+    const int D = p.head_dim, head = f_ / D, d = f_ - head * D;
+    f = f_;
+    pos0 = pos0_;
+    is_q = head < p.n_head;
+    const bool is_k = head < p.n_head + p.n_kv;
+    base = is_q ? static_cast<__nv_bfloat16*>(p.out) + f_
+                : static_cast<__nv_bfloat16*>(is_k ? p.kcache : p.vcache) +
+                      (long long)(head - p.n_head - (is_k ? 0 : p.n_kv)) * p.smax * D + d;
+  }
+  __device__ __forceinline__ void flush(const E2hGemmParams& p, const __nv_bfloat16* so, int et,
+                                        int t_first, int t_end) const {
+    if (f >= p.F) return;
+    int r = et >> 4, t = t_first + r;
+    int b = t / p.sq, s = t - b * p.sq;
+#pragma unroll
+    for (int u = 0; u < kChunkTok / 8; ++u, r += 8, t += 8) {
+      const int pos = pos0 + s;
+      if (t < t_end && (is_q || pos < p.smax)) {
+        const long long row = is_q ? (long long)t * p.ldo
+                                   : ((long long)b * p.n_kv * p.smax + pos) * p.head_dim;
+        *reinterpret_cast<uint4*>(base + row) =
+            *reinterpret_cast<const uint4*>(so + r * 128 + ((et & 15) << 3));
+      }
+      for (s += 8; s >= p.sq; s -= p.sq) ++b;
+    }
+  }
+};
+
 // PAIR: two CTAs of a cluster share one 256 (features) x 256 (tokens) tile with cta_group::2
 // instructions: CTA r of the pair owns features [128 r, 128 r + 128) of the tile (its A rows, its
 // accumulator lanes, its epilogue) and stages the B rows of tokens [128 r, 128 r + 128); the
 // leader (rank 0) issues every tcgen05.mma for both. The full barriers of the leader count the
 // TMA bytes of both CTAs, the commits are multicast to the barriers of both, and the peer's
 // epilogue warps hand the accumulator back on the leader's barrier.
-template <int BN, bool DUAL, bool PAIR>
+//
+// SWI: a pair tile whose 128 A rows per CTA are 64 rows of the gate matrix (lanes 0..63) above the
+// same 64 rows of the up matrix (lanes 64..127), so that a gated product runs on the same
+// 256 x 256 instructions, with the same operand bytes per instruction, as a plain one. The two
+// accumulators of a feature meet in the staging buffer of the epilogue (as bf16, which is what SwiGLU
+// rounds them to). Two accumulators of 128 x 128 side by side (DUAL) fetch 12 KB of operands for the
+// 64 cycles of tensor work that here cost 8 KB per 128: shared memory, not the tensor core, bounds
+// them. 16000 x 2 x 11008 x 4096: 2.24 -> 1.81 ms; 22432 x 2 x 22016 x 8192:
+// 14.6 -> 10.8 ms.
+template <int BN, bool DUAL, bool PAIR, bool SWI = false>
 __global__ void __launch_bounds__(kPThreads, 1)
 umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
                             const __grid_constant__ CUtensorMap tmA2,
@@ -133,6 +184,7 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
                             const __grid_constant__ CUtensorMap tmRes, const E2hGemmParams p,
                             const int staged, const int mn3d) {
   static_assert(!PAIR || (BN == 256 && !DUAL), "pair tiles are 2 x 128 features x 256 tokens");
+  static_assert(!SWI || PAIR, "gated pair tiles");
   constexpr int A_BYTES = 128 * 128;                  // 128 features x 64 k, bf16
   constexpr int BROWS = PAIR ? BN / 2 : BN;           // B rows staged by this CTA
   constexpr int B_BYTES = BROWS * 128;
@@ -152,7 +204,8 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
   const int crank = PAIR ? (int)cluster_ctarank() : 0;          // 0: leader of the pair
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;   // tile walker id
   const int n_workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  constexpr int TILE_F = PAIR ? 256 : 128;
+  constexpr int CTA_F = SWI ? 64 : 128;                 // output features of this CTA
+  constexpr int TILE_F = PAIR ? 2 * CTA_F : 128;
   const int n_f = (p.F + TILE_F - 1) / TILE_F, n_t = (p.T + BN - 1) / BN;
   int n_tiles = n_f * n_t;
   const int n_kb = (p.K + 63) / 64;
@@ -172,7 +225,7 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    if (DUAL) tma_prefetch_desc(&tmA2);
+    if (DUAL || SWI) tma_prefetch_desc(&tmA2);
     if (staged) tma_prefetch_desc(&tmOut);
   }
   if (warp == 1) {
@@ -222,7 +275,7 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     const uint32_t full_lead0 = PAIR ? mapa_shared(full0, 0) : full0;   // leader's full barriers
     for (int tile = worker; tile < n_tiles && ok; tile += n_workers) {
       const PTile pt = tile_at<BN>(p, ctrl, tile, n_f, n_t, grp);
-      const int f0 = pt.a_row + pt.ft * TILE_F + crank * 128;
+      const int f0 = pt.a_row + pt.ft * TILE_F + crank * CTA_F;
       const int t0 = pt.t0 + crank * BROWS * (PAIR ? 1 : 0);
       for (int kb = 0; kb < n_kb; ++kb, ++it) {
         if (!mbar_wait(empty0 + 8 * s, ph ^ 1, abort_flag, p.status, kStatusTimeoutEmpty)) {
@@ -236,7 +289,10 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
           const uint32_t bar = full_lead0 + 8 * s;
           if (crank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE);
           const int k0p = kb * 64;
-          if (!p.a_mn_major) {
+          if constexpr (SWI) {
+            tma_load_2d_pair(a_dst, &tmA, k0p, f0, bar);              // 64 rows of each matrix
+            tma_load_2d_pair(a_dst + A_BYTES / 2, &tmA2, k0p, f0, bar);
+          } else if (!p.a_mn_major) {
             tma_load_2d_pair(a_dst, &tmA, k0p, f0, bar);
           } else {
             tma_load_3d_pair(a_dst, &tmA, 0, k0p, f0 >> 6, bar);
@@ -360,8 +416,8 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
                                       : smem_u32(&ctrl->tmem_empty[0]);
     for (int tile = worker; tile < n_tiles; tile += n_workers, ++tcount) {
       const PTile pt = tile_at<BN>(p, ctrl, tile, n_f, n_t, grp);
-      const int f0 = pt.ft * TILE_F + crank * 128, t0 = pt.t0;
-      const int f = f0 + lane_row;
+      const int f0 = pt.ft * TILE_F + crank * CTA_F, t0 = pt.t0;
+      const int f = f0 + (SWI ? lane_row & 63 : lane_row);
       const int acc = tcount & 1;
       const uint32_t accph = (tcount >> 1) & 1;
       int ok_i = 1;
@@ -371,7 +427,51 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
       ok = ok && (__shfl_sync(0xffffffffu, ok_i, 0) != 0);
       tc_fence_after();
       const uint32_t a0 = taddr + acc * ACC_COLS;
-      if (staged) {
+      if constexpr (SWI) {
+        const int up = lane_row >> 6;                 // this lane's accumulator: gate or up
+        const float sc = (p.scale != nullptr && f < p.F) ? p.scale[up * p.F + f] : 1.f;
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
+        for (int c = 0; c < BN / kChunkTok; ++c, ++cc) {
+          float v[32];
+          if (ok) tmem_ld_x32p(a0 + c * kChunkTok, v);
+          tmem_ld_wait();
+          if (c + 1 == BN / kChunkTok) {   // accumulator fully read: hand it back to the MMA
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(tmem_empty0 + 8 * acc);
+          }
+          // [token][64 gate | 64 up]. The two buffers alternate: whoever is past the barrier of a
+          // chunk has read the buffer that the next chunk fills
+          __nv_bfloat16* so = reinterpret_cast<__nv_bfloat16*>(stage_out + (cc & 1) * kChunkBytes);
+#pragma unroll
+          for (int j = 0; j < kChunkTok; ++j) so[j * 128 + lane_row] = __float2bfloat16_rn(v[j] * sc);
+          epi_bar_sync();
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = et + u * 128, r = i >> 3, fv = (i & 7) << 3;
+            const int t = t0 + c * kChunkTok + r;
+            if (ok && t < pt.t_end && f0 + fv < p.F) {
+              const uint4 gq = *reinterpret_cast<const uint4*>(so + r * 128 + fv);
+              const uint4 uq = *reinterpret_cast<const uint4*>(so + r * 128 + 64 + fv);
+              const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gq);
+              const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&uq);
+              uint4 res;
+              __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&res);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 g = __bfloat1622float2(g2[k]), w = __bfloat1622float2(u2[k]);
+                o2[k] = __floats2bfloat162_rn(bf16_round(silu(g.x)) * w.x,
+                                              bf16_round(silu(g.y)) * w.y);
+              }
+              *reinterpret_cast<uint4*>(out + (long long)t * p.ldo + f0 + fv) = res;
+            }
+          }
+        }
+      } else if (staged) {
+        const bool rope = p.epi == E2H_EPI_ROPE_KV;
+        const RopePre rp = rope ? rope_prepare(p, f) : RopePre();
+        RopeRows rope_rows;
+        if (rope && p.kcache != nullptr) rope_rows.prepare(p, rp.pos0, f0 + ((et & 15) << 3));
         if (with_res && et == 0 && ok) {   // first residual chunk of the tile
           const int b = cc & 1;
           mbar_expect_tx(smem_u32(&ctrl->res_full[b]), kChunkBytes);
@@ -393,6 +493,10 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
           if (ok) {
             tmem_ld_x32p(a0 + c * kChunkTok, v);
             if constexpr (DUAL) tmem_ld_x32p(a0 + BN + c * kChunkTok, v2);
+          }
+          __nv_bfloat162 cs[kChunkTok];
+          if constexpr (!DUAL) {
+            if (rope) rope_factors<kChunkTok>(p, rp, f, t0 + c * kChunkTok, pt.t_end, cs);
           }
           tmem_ld_wait();
           if (c + 1 == BN / kChunkTok) {   // accumulator fully read: hand it back to the MMA
@@ -440,6 +544,20 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           const __nv_bfloat16* sr =
               reinterpret_cast<const __nv_bfloat16*>(stage_res + b * kChunkBytes);
+          if constexpr (!DUAL) {
+            if (rope) {
+              const float sign = (rp.d & 1) ? 1.f : -1.f;
+#pragma unroll
+              for (int j = 0; j < kChunkTok; ++j) {
+                const float x = bf16_round(v[j] * sc);
+                const float partner = __shfl_xor_sync(0xffffffffu, x, 1);
+                const float2 r = __bfloat1622float2(cs[j]);
+                so[j * 128 + lane_row] =
+                    __float2bfloat16_rn(rp.is_v ? x : x * r.x + sign * (partner * r.y));
+              }
+            }
+          }
+          if (DUAL || !rope) {
 #pragma unroll
           for (int j = 0; j < kChunkTok; ++j) {
             float y;
@@ -452,8 +570,13 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
             }
             so[j * 128 + lane_row] = __float2bfloat16_rn(y);
           }
+          }
           fence_proxy_async_smem();
           epi_bar_sync();
+          if (rope && p.kcache != nullptr) {   // query rows and cache rows, 16 bytes at a time
+            if (ok) rope_rows.flush(p, so, et, t0 + c * kChunkTok, pt.t_end);
+            continue;
+          }
           if (p.n_groups > 0) {
             // the rows behind the group belong to the next one: bounded 16-byte stores
             __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
@@ -585,7 +708,7 @@ static int p_map_mn3d(CUtensorMap* m, const void* base, long long mn, long long 
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-template <int BN, bool DUAL, bool PAIR>
+template <int BN, bool DUAL, bool PAIR, bool SWI = false>
 static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
   constexpr int BROWS = PAIR ? BN / 2 : BN;
   constexpr int STAGE = 128 * 128 * (DUAL ? 2 : 1) + BROWS * 128;
@@ -598,11 +721,11 @@ static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
     r = p_map_mn3d(&ta, p.a, p.F, p.K, p.lda, 2);
   } else {
     r = p.a_mn_major ? p_map(&ta, p.a, p.F, p.K, p.lda, 64, 64, true)
-                     : p_map(&ta, p.a, p.K, a_rows, p.lda, 64, 128, true);
+                     : p_map(&ta, p.a, p.K, a_rows, p.lda, 64, SWI ? 64 : 128, true);
   }
   if (r) return r;
-  if (DUAL) {
-    r = p_map(&ta2, p.a2, p.K, a_rows, p.lda2, 64, 128, true);
+  if (DUAL || SWI) {
+    r = p_map(&ta2, p.a2, p.K, a_rows, p.lda2, 64, SWI ? 64 : 128, true);
     if (r) return r;
   } else {
     ta2 = ta;
@@ -616,7 +739,8 @@ static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
   }
   if (r) return r;
   int staged = (p.epi == E2H_EPI_STORE_BF16 || p.epi == E2H_EPI_RESIDUAL ||
-                (p.epi == E2H_EPI_SWIGLU && DUAL)) ? 1 : 0;
+                (p.epi == E2H_EPI_SWIGLU && DUAL) ||
+                (p.epi == E2H_EPI_ROPE_KV && epi_can_stage(p, 128))) ? 1 : 0;
   if (staged && p.n_groups > 0 && (p.F % 8)) staged = 0;
   if (staged && ((p.ldo % 8) || ((uintptr_t)p.out & 15))) staged = 0;
   if (staged && p.epi == E2H_EPI_RESIDUAL && ((uintptr_t)p.aux & 15)) staged = 0;
@@ -646,7 +770,7 @@ static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
   if (stages < 2) return -8;
   p.stages = stages;
   const size_t smem = 2048 + (size_t)stages * STAGE + 4 * kChunkBytes;
-  auto kern = umma_gemm_persistent_kernel<BN, DUAL, PAIR>;
+  auto kern = umma_gemm_persistent_kernel<BN, DUAL, PAIR, SWI>;
   static size_t configured = 0;
   if (smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -666,7 +790,8 @@ static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
   }
   if constexpr (PAIR) {
     // one cluster of two CTAs per 256 x 256 tile walker
-    const int n_tiles = (p.F / 256) * ((p.T + BN - 1) / BN + p.n_groups);
+    constexpr int TILE_F = SWI ? 128 : 256;
+    const int n_tiles = ((p.F + TILE_F - 1) / TILE_F) * ((p.T + BN - 1) / BN + p.n_groups);
     const int pairs = n_tiles < n_sm / 2 ? n_tiles : n_sm / 2;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -717,11 +842,15 @@ extern "C" int e2h_gemm_persistent(const E2hGemmParams* pp, void* stream_v) {
   if (p.dual && (p.a_mn_major || p.a2 == nullptr)) return -5;
   if ((p.lda % 8) || (p.ldb % 8) || (p.dual && (p.lda2 % 8))) return -6;
   if (((uintptr_t)p.a & 15) || ((uintptr_t)p.b & 15)) return -7;
+  // tf == 256 asks for CTA-pair tiles (cta_group::2)
+  if (p.dual && p.tf == 256 && p.bn == 256 && p.epi == E2H_EPI_SWIGLU && (p.K % 64) == 0 &&
+      (p.F % 8) == 0 && (p.ldo % 8) == 0 && ((uintptr_t)p.out & 15) == 0 && p.n_signal == 0)
+    return p_launch<256, false, true, true>(p, stream);
   if (p.dual) return p_launch<128, true, false>(p, stream);
   if (p.bn == 128) return p_launch<128, false, false>(p, stream);
-  // tf == 256 asks for CTA-pair tiles (cta_group::2): 256-feature tiles, operands that the 3-D
-  // boxes can address
-  if (p.tf == 256 && (p.F % 256) == 0 && p.T > 256 && (p.K % 64) == 0 &&
+  // 256-feature tiles, operands that the 3-D boxes can address. A last tile that reaches past F
+  // reads zeros (or, in a grouped product, rows of the next matrix) and masks its stores
+  if (p.tf == 256 && (!p.a_mn_major || (p.F % 256) == 0) && p.T > 256 && (p.K % 64) == 0 &&
       (!p.b_mn_major || (p.T % 64) == 0))
     return p_launch<256, false, true>(p, stream);
   return p_launch<256, false, false>(p, stream);

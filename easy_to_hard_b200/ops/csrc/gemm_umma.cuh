@@ -47,7 +47,8 @@ struct E2hGemmParams {
   const int* pos_base;   // device scalar: cache position of the first token of every sequence
   int sq;                // tokens per sequence in this call (1 for decode)
   int n_head, n_kv, head_dim, smax;
-  void* kcache;          // bf16 [max_batch, n_kv, smax, head_dim]
+  void* kcache;          // bf16 [max_batch, n_kv, smax, head_dim]; null: keys and values stay in
+                         // `out` beside the queries (smax is then the length of `freqs`)
   void* vcache;
   int* status;           // int32 status word (0 = ok)
   int tf;                // features per tile: 128 (default) or 64 (more CTAs for skinny GEMMs)

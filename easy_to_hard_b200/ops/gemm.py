@@ -258,7 +258,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         p.sq = rope["sq"]
         p.n_head, p.n_kv, p.head_dim = rope["n_head"], rope["n_kv"], rope["head_dim"]
         p.smax = rope["smax"]
-        p.kcache, p.vcache = rope["kcache"].data_ptr(), rope["vcache"].data_ptr()
+        if rope["kcache"] is not None:
+            p.kcache, p.vcache = rope["kcache"].data_ptr(), rope["vcache"].data_ptr()
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() >= F
         p.bias = bias.data_ptr()
@@ -283,8 +284,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
            (T > bn and splitk == 1 and tf == 128 and tiled_shape is None
             and bn >= 128))
     if big:
-        if (pair if pair is not None else PAIR_DEFAULT) and not dual and bn == 256:
-            p.tf = 256      # CTA-pair (cta_group::2) tiles where the shape allows them
+        if pair if pair is not None else PAIR_DEFAULT:
+            # CTA-pair (cta_group::2) tiles where the shape allows them. Gated products get them
+            # from two 128-token tiles a group on: below, half of the 256-token tiles is padding
+            if dual and epi == EPI_SWIGLU and not b_mn_major and T >= 256 * max(1, n_groups):
+                p.tf, p.bn = 256, 256
+            elif not dual and bn == 256:
+                p.tf = 256
         _lib.check(_lib.lib().e2h_gemm_persistent(C.byref(p), _lib.stream()),
                    "e2h_gemm_persistent")
     else:
@@ -438,14 +444,17 @@ def linear_dual(x, w1, w3, out1=None, out2=None, **kw):
     return out1, out2
 
 
-def linear_qkv_rope(x, wqkv, q_out, *, freqs, pos_base, sq, n_head, n_kv, head_dim, kcache,
-                    vcache, **kw):
+def linear_qkv_rope(x, wqkv, q_out, *, freqs, pos_base, sq, n_head, n_kv, head_dim, kcache=None,
+                    vcache=None, **kw):
     """Fused QKV projection + RoPE(q, k) + scatter of k, v into the static KV cache.
 
     q_out [T, n_head*head_dim]; caches [max_batch, n_kv, smax, head_dim]; token t belongs to
-    sequence t // sq and sits at cache position pos_base + t % sq."""
+    sequence t // sq and sits at cache position pos_base + t % sq. Without caches, keys and values
+    follow the queries in q_out [T, (n_head + 2 n_kv) * head_dim]."""
+    assert kcache is not None or q_out.shape[1] == (n_head + 2 * n_kv) * head_dim
     rope = dict(freqs=freqs, pos_base=pos_base, sq=sq, n_head=n_head, n_kv=n_kv,
-                head_dim=head_dim, smax=kcache.shape[2], kcache=kcache, vcache=vcache)
+                head_dim=head_dim, smax=freqs.shape[0] if kcache is None else kcache.shape[2],
+                kcache=kcache, vcache=vcache)
     gemm(wqkv, x, epi=EPI_ROPE_KV, out=q_out, rope=rope, **kw)
     return q_out
 

@@ -200,3 +200,91 @@ def test_stream_tiles_dual_swiglu(T, F, K):
     g = (x.float() @ w1.float().t()).bfloat16().float()
     u = (x.float() @ w3.float().t()).bfloat16().float()
     _close(y, torch.nn.functional.silu(g).bfloat16().float() * u)
+
+
+@pytest.mark.parametrize("cache", [True, False])
+@pytest.mark.parametrize("sq,B,n_head,n_kv,D", [(130, 3, 8, 2, 64), (257, 2, 2, 1, 128),
+                                                 (31, 17, 6, 2, 64), (1, 300, 4, 4, 64)])
+def test_qkv_rope_many_tokens(sq, B, n_head, n_kv, D, cache):
+    """The staged RoPE epilogue of the persistent tiles: sequences that start and end inside a
+    32-token chunk, tiles across query / key / value heads, features off the 256-feature grid,
+    cache rows or (without caches) all rows behind the queries. Rounding: the fp32 sum and its
+    rotation may each differ by one bf16 step (2^-8 of the largest value)."""
+    from easy_to_hard_b200.ops import gemm, reference
+    dim, smax, pos0, T = 512, 272, 5, B * sq
+    x = _mk(T, dim, seed=47)
+    w = _mk((n_head + 2 * n_kv) * D, dim, scale=1 / math.sqrt(dim), seed=48)
+    freqs = reference.precompute_freqs_cis(smax, D, 10000.0, device="cuda")
+    pos = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+    kw = dict(freqs=freqs, pos_base=pos, sq=sq, n_head=n_head, n_kv=n_kv, head_dim=D)
+    qkv = (x.float() @ w.float().T).bfloat16().view(B, sq, -1)
+    want = [t.reshape(B, sq, -1, D) for t in qkv.split([n_head * D, n_kv * D, n_kv * D], -1)]
+    want[:2] = [reference.apply_rotary_emb(t, freqs[pos0:pos0 + sq]) for t in want[:2]]
+    if cache:
+        kc = torch.zeros(B + 1, n_kv, smax, D, dtype=torch.bfloat16, device="cuda")
+        vc, q = torch.zeros_like(kc), torch.empty(T, n_head * D, dtype=torch.bfloat16, device="cuda")
+        gemm.linear_qkv_rope(x, w, q, kcache=kc, vcache=vc, **kw)
+        got = [q.view(B, sq, n_head, D)] + [c[:B, :, pos0:pos0 + sq].transpose(1, 2)
+                                            for c in (kc, vc)]
+        for c in (kc, vc):
+            assert not c[B].any() and not c[:, :, :pos0].any() and not c[:, :, pos0 + sq:].any()
+    else:
+        out = torch.empty(T, w.shape[0], dtype=torch.bfloat16, device="cuda")
+        gemm.linear_qkv_rope(x, w, out, **kw)
+        got = [t.reshape(B, sq, -1, D) for t in out.split([n_head * D, n_kv * D, n_kv * D], -1)]
+    _check_status()
+    for g, r in zip(got, want):
+        _close(g, r, rtol=2 ** -7, atol=2 ** -8 * float(r.abs().max()))
+
+
+@pytest.mark.parametrize("T,F,K", [(256, 136, 64), (300, 688, 512), (1000, 1376, 192),
+                                   (515, 128, 1088)])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_gated_pair_tiles(T, F, K, scaled):
+    """SwiGLU on pair tiles of 64 gate and 64 up rows per CTA: features off the tile grid, ragged
+    tokens, per-feature scales of both matrices. One bf16 step on each factor and on the result."""
+    from easy_to_hard_b200.ops import gemm
+    x = _mk(T, K, seed=49)
+    w1, w3 = _mk(F, K, scale=1 / math.sqrt(K), seed=50), _mk(F, K, scale=1 / math.sqrt(K), seed=51)
+    s = torch.rand(2 * F, device="cuda") + 0.5 if scaled else torch.ones(2 * F, device="cuda")
+    out = torch.full((T, F + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.linear_swiglu(x, w1, w3, out=out[:, :F], **(dict(scale=s) if scaled else {}))
+    _check_status()
+    g = (x.float() @ w1.float().T * s[:F]).bfloat16()
+    u = (x.float() @ w3.float().T * s[F:]).bfloat16()
+    want = (torch.nn.functional.silu(g) * u).float()
+    _close(out[:, :F], want, rtol=2 ** -6, atol=2 ** -7 * float(want.abs().max()))
+    assert bool((out[:, F:] == 7.0).all())
+
+
+def test_gated_pair_tiles_of_groups():
+    from easy_to_hard_b200.ops import gemm
+    sizes, F, K = [0, 300, 1, 700, 255], 200, 128
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    T, n = 1300, len(sizes)
+    x = _mk(T, K, seed=52)
+    w1, w3 = _mk(n * F, K, scale=0.1, seed=53), _mk(n * F, K, scale=0.1, seed=54)
+    out = torch.zeros(T, F, dtype=torch.bfloat16, device="cuda")
+    gemm.grouped_swiglu(x, w1, w3, out, off, n, 1300)
+    _check_status()
+    for i in range(n):
+        a, b = int(off[i]), int(off[i + 1])
+        g, u = ((x[a:b].float() @ w[i * F:(i + 1) * F].float().T).bfloat16() for w in (w1, w3))
+        if b > a:
+            want = (torch.nn.functional.silu(g) * u).float()
+            _close(out[a:b], want, rtol=2 ** -6, atol=2 ** -7 * float(want.abs().max()))
+    assert not out[int(off[-1]):].any()
+
+
+@pytest.mark.parametrize("T,F,K", [(515, 640, 1088), (300, 136, 128), (1024, 1000, 64)])
+def test_cta_pair_tiles_past_the_features(T, F, K):
+    """A last pair tile that is only partly inside F: zero-filled rows, masked stores."""
+    from easy_to_hard_b200.ops import gemm
+    x, w, r = _mk(T, K, seed=55), _mk(F, K, scale=1 / math.sqrt(K), seed=56), _mk(T, F, seed=57)
+    want = x.float() @ w.float().T
+    _close(gemm.linear(x, w, pair=True), want, rtol=2 ** -7, atol=2 ** -8 * float(want.abs().max()))
+    y = gemm.linear(x, w, out_dtype=torch.float32, pair=True)
+    _close(y, want, rtol=1e-4, atol=1e-4)       # fp32 sums of bf16 products, in another order
+    _close(gemm.linear_residual(x, w, r, pair=True), want.bfloat16().float() + r.float(),
+           rtol=2 ** -7, atol=2 ** -7 * float(want.abs().max()))
+    _check_status()
