@@ -369,7 +369,12 @@ def _expand_int8(w: torch.Tensor, which: int) -> torch.Tensor:
         buf = torch.empty(w.numel(), dtype=torch.bfloat16, device=w.device)
         _INT8_SCRATCH[key] = buf
     out = buf[: w.numel()].view(w.shape)
-    out.copy_(w)
+    F, K = w.shape
+    if K % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 8 == 0:
+        _lib.check(_lib.lib().e2h_expand_weight(w.data_ptr(), w.stride(0), 8, None, 0, out.data_ptr(),
+                                                F, K, _lib.stream()), "e2h_expand_weight")
+    else:
+        out.copy_(w)
     return out
 
 
@@ -382,7 +387,13 @@ def _expand_int4(w: "Int4Weight", which: int) -> torch.Tensor:
         buf = torch.empty(n, dtype=torch.bfloat16, device=w.device)
         _INT8_SCRATCH[key] = buf
     out = buf[:n].view(w.shape)
-    out.copy_(w.dequant())
+    F, K = w.shape
+    if w.groupsize % 8 == 0 and w.q.stride(1) == 1 and w.q.stride(0) % 4 == 0:
+        _lib.check(_lib.lib().e2h_expand_weight(w.q.data_ptr(), w.q.stride(0), 4, w.sz.data_ptr(),
+                                                w.groupsize, out.data_ptr(), F, K, _lib.stream()),
+                   "e2h_expand_weight")
+    else:
+        out.copy_(w.dequant())
     return out
 
 
