@@ -149,6 +149,7 @@ _SIGNATURES = {
     "e2h_gemm_w8": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_w4": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_f32": [C.POINTER(GemmParams), _vp],
+    "e2h_gemm_rows": [C.POINTER(GemmParams), _i, _vp],
     "e2h_expand_weight": [_vp, _ll, _i, _vp, _i, _vp, _i, _i, _vp],
     "e2h_stream_norm": [C.POINTER(StreamNormParams), _i, _i, _vp],
     "e2h_attn_prep": [C.POINTER(AttnWindowParams), _i, _vp],

@@ -244,7 +244,7 @@ __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0,
         }
         cj[j] = 1.f;
         sj[j] = 0.f;
-        if (!is_v && f_ok && t0 + j < t_end) {
+        if (!is_v && f_ok && t0 + j < t_end && posj[j] >= 0 && posj[j] < p.smax) {
           const __nv_bfloat162 cs = freqs2[(long long)posj[j] * (D / 2) + (d >> 1)];
           cj[j] = __bfloat162float(cs.x);
           sj[j] = __bfloat162float(cs.y);
@@ -261,7 +261,7 @@ __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0,
         const __nv_bfloat16 yb = __float2bfloat16_rn(y);
         if (is_q || p.kcache == nullptr) {
           static_cast<__nv_bfloat16*>(p.out)[(long long)t * p.ldo + f] = yb;
-        } else if (posj[j] < p.smax) {
+        } else if (posj[j] >= 0 && posj[j] < p.smax) {
           cache[(((long long)bj[j] * p.n_kv + hk) * p.smax + posj[j]) * D + d] = yb;
         }
       }

@@ -101,6 +101,33 @@ def pick_stream_tiles(F: int, K: int, bn: int, dual: bool):
     return th
 
 
+ROWS_EPIS = {EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_RESIDUAL_F32, EPI_ROPE_KV}
+ROWS_GATED = {EPI_SWIGLU, EPI_DUAL_STORE}
+ROWS_MAX = 16
+
+
+def rows_rule(a, a2, b, epi: int) -> bool:
+    """Whether a product runs on the kernel for few rows (csrc/gemm_rows.cu): up to 16, the range that
+    its two groups of eight token columns cover and over which it is nowhere slower than the tcgen05
+    kernels (16 rows, 4096 x 11008: 21.8 us both; everything smaller gains, by up to 3x), token-major
+    outputs, and operands whose rows are whole 16-byte pieces. Anything else goes where it went."""
+    T, K = b.shape
+    if T > ROWS_MAX or epi not in (ROWS_EPIS if a2 is None else ROWS_GATED):
+        return False
+    if _ld(b) % 8 or b.data_ptr() % 16:
+        return False
+    for w in (a,) if a2 is None else (a, a2):
+        if isinstance(w, Int4Weight):
+            q, piece, g = w.q, 128, w.groupsize
+            if g < 32 or g & (g - 1):
+                return False
+        else:
+            q, piece = w, 16 // w.element_size()
+        if K % piece or _ld(q) * q.element_size() % 16 or q.data_ptr() % 16:
+            return False
+    return True
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tensor] = None,
          a2: Optional[torch.Tensor] = None, out2: Optional[torch.Tensor] = None,
          aux: Optional[torch.Tensor] = None, scale: Optional[torch.Tensor] = None,
@@ -128,12 +155,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
     matrix first for larger token counts."""
     assert a.is_cuda and b.is_cuda and b.dtype == torch.bfloat16
     w4 = isinstance(a, Int4Weight)
+    rows = (not (a_mn_major or b_mn_major or n_groups or signal or stages) and tiled_shape is None
+            and batch is None and splitk is None and bn is None and tf is None and th is None
+            and kps <= 0 and persistent is None and pair is None and rows_rule(a, a2, b, epi))
     if w4:
         assert not a_mn_major and not b_mn_major and tiled_shape is None and scale is None
         assert a2 is None or isinstance(a2, Int4Weight)
         K4 = a.shape[1]
-        if (b.shape[0] > 128 or K4 % 128 or a.groupsize < 64 or a.groupsize & (a.groupsize - 1)
-                or (K4 // 2) % 16):
+        if not rows and (b.shape[0] > 128 or K4 % 128 or a.groupsize < 64 or a.groupsize & (a.groupsize - 1)
+                         or (K4 // 2) % 16):
             a = _expand_int4(a, 0)            # many tokens: one dequantisation pass, then bf16
             a2 = _expand_int4(a2, 1) if a2 is not None else None
             w4 = False
@@ -142,7 +172,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         assert scale is not None and not a_mn_major and not b_mn_major and tiled_shape is None
         if a2 is not None:
             assert a2.dtype == torch.int8
-        if b.shape[0] > 128 or a.shape[1] % 128 or _ld(a) % 16:
+        if not rows and (b.shape[0] > 128 or a.shape[1] % 128 or _ld(a) % 16):
             a = _expand_int8(a, 0)
             a2 = _expand_int8(a2, 1) if a2 is not None else None
             w8 = False
@@ -272,6 +302,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         assert group_off.dtype == torch.int32 and group_off.numel() > n_groups
         p.n_groups, p.group_tmax, p.group_off = n_groups, group_tmax, group_off.data_ptr()
     p.status = _lib.status_word(a.device).data_ptr()
+    if rows:
+        _lib.check(_lib.lib().e2h_gemm_rows(C.byref(p), 4 if w4 else 8 if w8 else 16, _lib.stream()),
+                   "e2h_gemm_rows")
+        return
     # more than one token tile: the persistent kernel (double-buffered accumulator, TMA-store
     # epilogue); skinny / split-K shapes: the latency-oriented one-tile-per-CTA kernel
     if w8:
