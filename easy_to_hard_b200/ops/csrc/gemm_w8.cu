@@ -44,7 +44,7 @@ constexpr int kW8Threads = 320;     // TMA warp, MMA warp, 8 converter warps (4 
 constexpr int kW8MaxStages = 8;
 constexpr int kW8Ctrl = 1024;
 constexpr int kW8Kps = 2;          // 64-wide k-blocks per pipeline stage
-constexpr int kW8ConvMax = 4;      // converted-tile buffers: 4 (2 for a dual GEMM, whose tiles are twice as large)
+constexpr int kW8ConvMax = 4;      // converted-tile buffers: 4 (3 for a dual GEMM, whose tiles are twice as large)
 constexpr int kW8ACol0 = 128;      // tensor-memory column of the first converted-tile buffer
 constexpr int kW8ACols = 64;       // columns of one converted [128 x 128 k] bf16 tile
 constexpr int kW8TmemCols = 512;
@@ -74,8 +74,8 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int NMAT = DUAL ? 2 : 1;
   // the conversion -> MMA -> commit round trip of one buffer takes about 2 us; several buffers
   // in flight hide it. Tensor memory: accumulators in columns [0, 128), converted tiles in
-  // [128, 384): 4 buffers of 64 columns (2 of 128 for a dual GEMM).
-  constexpr int kW8Conv = DUAL ? 2 : 4;
+  // [128, 512): 4 buffers of 64 columns (3 of 128 for a dual GEMM).
+  constexpr int kW8Conv = DUAL ? 3 : 4;
   constexpr int B_BYTES = BN * 128;
   // quantised weight tile of one stage: TH rows x 128 k. TH = p.th (64..128): with lower tiles
   // a wide layer covers (nearly) all SMs in one wave instead of leaving a third of them idle;
@@ -138,7 +138,7 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   // it waits for the predecessor, every other thread that touches global memory waits first
   pdl_launch_dependents();
   const bool early_weights = true;
-  if (!(warp == 0 && lane == 0 && early_weights) && !(warp == 1 && lane == 0)) pdl_wait_prior();
+  if (!(warp == 0 && lane == 0 && early_weights) && warp != 1) pdl_wait_prior();
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer ----------------
@@ -192,49 +192,58 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- UMMA issuer ----------------
+    // The whole warp walks the loop and one lane issues: the operands of an instruction are then
+    // uniform values. In a branch of a single lane an instruction took 66 to 88 cycles to issue (64
+    // rows) where the tensor core takes 32, and the wait for the stage's own barrier another 220 per
+    // stage. 2 x 11008 x 4096 int8, 64 rows, one launch: 52.7 -> 48.2 us; 12288 x 4096: 32.1 -> 28.3.
+    // What is left is the converters' instruction issue.
+    const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, BN, 0, 0);
     // descriptors: constant high word, base low words once, one add per instruction; stage and
     // phase are running counters (no division in this dependent scalar chain)
     const uint32_t d_hi = sw128_desc_hi(1024);
+    const uint32_t d0 = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t b_lo0 = sw128_desc_lo(smem_u32(tiles) + AQ_BYTES * NMAT, 16);
-    const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
+    const uint32_t empty0 = smem_u32(&ctrl->empty[0]);
+    const uint32_t cfull0 = smem_u32(&ctrl->conv_full[0]), cempty0 = smem_u32(&ctrl->conv_empty[0]);
+    int s = 0, c = 0;
+    uint32_t cph = 0, st_lo = 0;
     bool ok = true;
-    int s = 0;
-    uint32_t ph = 0, st_lo = 0, accf = 0;
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int c = it % kW8Conv;
-      ok = mbar_wait(full0 + 8 * s, ph, abort_flag, p.status, kStatusTimeoutFull) &&
-           mbar_wait(smem_u32(&ctrl->conv_full[c]), (it / kW8Conv) & 1, abort_flag, p.status,
-                     kStatusTimeoutFull);
+    for (int it = 0; it < n_it; ++it) {
+      // (the converters have seen the stage's full barrier before they arrive here)
+      ok = __all_sync(0xffffffffu, mbar_wait(cfull0 + 8 * c, cph, abort_flag, p.status,
+                                             kStatusTimeoutFull));
       if (!ok) break;
       tc_fence_after();
-      const int kcount = min(kW8Kps, n_kb - it * kW8Kps);
       // A: 8 columns (16 k) per instruction, 32 columns per 64-wide k block
-      uint32_t a_col = tmem_base + kW8ACol0 + c * CONV_COLS, b_lo = b_lo0 + st_lo;
-      for (int kk = 0; kk < kcount; ++kk) {
+      const uint32_t a_col = d0 + kW8ACol0 + c * CONV_COLS, b_lo = b_lo0 + st_lo;
+      if (lead) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          umma_f16_ts(tmem_base, a_col + 8 * k, b_lo + 2 * k, d_hi, idesc, accf);
+        for (int k = 0; k < 4 * kW8Kps; ++k) {
+          const uint32_t bk = b_lo + (k >> 2) * (B_BYTES >> 4) + 2 * (k & 3);
+          umma_f16_ts(d0, a_col + 8 * k, bk, d_hi, idesc, k > 0 || it > 0);
           if (DUAL)
-            umma_f16_ts(tmem_base + BN, a_col + kW8ACols + 8 * k, b_lo + 2 * k, d_hi, idesc, accf);
-          accf = 1;
+            umma_f16_ts(d0 + BN, a_col + kW8ACols + 8 * k, bk, d_hi, idesc, k > 0 || it > 0);
         }
-        a_col += 32;
-        b_lo += B_BYTES >> 4;
+        umma_commit(empty0 + 8 * s);                   // activation tile (and int8 tile) reusable
+        umma_commit(cempty0 + 8 * c);                  // converted tile reusable
       }
-      umma_commit(empty0 + 8 * s);                   // activation tile (and int8 tile) reusable
-      umma_commit(smem_u32(&ctrl->conv_empty[c]));   // converted tile reusable
+      __syncwarp();
+      if (++c == kW8Conv) {
+        c = 0;
+        cph ^= 1;
+      }
       if (++s == stages) {
         s = 0;
         st_lo = 0;
-        ph ^= 1;
       } else {
         st_lo += STAGE >> 4;
       }
     }
-    umma_commit(smem_u32(&ctrl->tmem_full));
+    if (lead) umma_commit(smem_u32(&ctrl->tmem_full));
+    __syncwarp();
   }
 
   const bool is_conv = warp >= 2;
