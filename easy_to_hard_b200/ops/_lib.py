@@ -51,6 +51,7 @@ class GemmParams(C.Structure):
         ("n_groups", C.c_int), ("group_tmax", C.c_int), ("group_off", C.c_void_p),
         ("out_scale", C.c_float), ("softcap", C.c_float),
         ("n_batch", C.c_int), ("batch_k", C.c_int), ("batch_out", C.c_int),
+        ("early", C.c_int),
     ]
 
 

@@ -61,10 +61,11 @@ __device__ __forceinline__ void store_tail(const E2hGemmParams& p, int f, int t0
 // Applies the epilogue to 8 consecutive token columns of one feature. Tokens from t_end on are
 // masked (p.T, or the end of the group in a grouped product); o_col: first output column of this
 // matrix of a batched product.
-template <bool DUAL>
+template <bool DUAL, int EPI = -1>
 __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0, float* v,
                                           float* v2, int t_end, int o_col = 0) {
   const bool f_ok = f < p.F;
+  const int epi = EPI >= 0 ? EPI : p.epi;
   if (p.scale != nullptr) {
     const float s = f_ok ? p.scale[f] : 0.f;
 #pragma unroll
@@ -75,7 +76,7 @@ __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0,
       for (int j = 0; j < 8; ++j) v2[j] *= s2;
     }
   }
-  switch (p.epi) {
+  switch (epi) {
     case E2H_EPI_STORE_BF16: {
       __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
       if (!f_ok) break;
@@ -280,6 +281,10 @@ __device__ __forceinline__ void epilogue8(const E2hGemmParams& p, int f, int t0,
 // warps then move the tile with 16-byte accesses, 8 consecutive features of one token per
 // thread (flush_tile): full 32-byte sectors, and the residual is read the same way.
 
+// EPI >= 0 in these functions: the epilogue is known at compile time, and a RoPE launch has one token
+// per sequence (decode). In a chain of short kernels straight-line code runs from a cold instruction
+// cache, so what a launch does not need should not lie between what it does.
+
 // True when this launch can take the staged path: bf16 token-major output whose rows and tile
 // origins are 16-byte aligned.
 __host__ __device__ inline bool epi_can_stage(const E2hGemmParams& p, int tile_rows) {
@@ -346,11 +351,12 @@ __device__ __forceinline__ void rope_factors(const E2hGemmParams& p, const RopeP
 // tile[(tl + j) * pitch + row] for j < 8 (row < 0: a lane without a feature, nothing is
 // written). The residual of E2H_EPI_RESIDUAL is added by flush_tile. All 32 lanes must call
 // (the RoPE partner value comes from the neighbouring lane).
-template <bool DUAL>
+template <bool DUAL, int EPI = -1>
 __device__ __forceinline__ void stage8(const E2hGemmParams& p, int f, int t0, float* v, float* v2,
                                        __nv_bfloat16* tile, int tl, int pitch, int row,
                                        const RopePre* rope, int t_end) {
   const bool f_ok = f < p.F;
+  const int epi = EPI >= 0 ? EPI : p.epi;
   if (p.scale != nullptr) {
     const float s = f_ok ? p.scale[f] : 0.f;
 #pragma unroll
@@ -362,15 +368,15 @@ __device__ __forceinline__ void stage8(const E2hGemmParams& p, int f, int t0, fl
     }
   }
   float y[8];
-  if (p.epi == E2H_EPI_SWIGLU) {
+  if (epi == E2H_EPI_SWIGLU) {
     if constexpr (DUAL) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) y[j] = bf16_round(silu(bf16_round(v[j]))) * bf16_round(v2[j]);
     }
-  } else if (p.epi == E2H_EPI_ROPE_KV) {
+  } else if (epi == E2H_EPI_ROPE_KV) {
     const RopePre rp = rope ? *rope : rope_prepare(p, f);
     const int D = p.head_dim;
-    if (p.sq == 1) {
+    if (EPI >= 0 || p.sq == 1) {
       // decode: every token sits at cache position pos0
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -399,7 +405,7 @@ __device__ __forceinline__ void stage8(const E2hGemmParams& p, int f, int t0, fl
       }
     }
   } else {
-    if (p.epi == E2H_EPI_STORE_BF16 && f_ok) {
+    if (epi == E2H_EPI_STORE_BF16 && f_ok) {
       bias_act<8>(p, f, v);
       if (in_tail(p, f)) {
         if (row >= 0) store_tail<8>(p, f, t0, v, t_end);
@@ -417,13 +423,16 @@ __device__ __forceinline__ void stage8(const E2hGemmParams& p, int f, int t0, fl
 // Moves the staged tile (rows = tokens t_first .. t_first + n_tok, columns = features f_first ..
 // f_first + pitch) to its destination, 16 bytes per access. `tid` / `nthreads`: the calling
 // thread's index among the epilogue threads, which have synchronised after stage8.
+template <int EPI = -1>
 __device__ __forceinline__ void flush_tile(const E2hGemmParams& p, const __nv_bfloat16* tile,
                                            int pitch, int f_first, int t_first, int n_tok,
                                            int tid, int nthreads, int t_end, int o_col = 0) {
+  const int epi = EPI >= 0 ? EPI : p.epi;
+  const int sq = EPI >= 0 ? 1 : p.sq;
   const int vpr = pitch >> 3;
   const int total = n_tok * vpr;
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
-  const int pos0 = (p.epi == E2H_EPI_ROPE_KV) ? *p.pos_base : 0;
+  const int pos0 = (epi == E2H_EPI_ROPE_KV) ? *p.pos_base : 0;
   for (int i = tid; i < total; i += nthreads) {
     const int r = i / vpr;
     const int fv = (i - r * vpr) << 3;
@@ -431,7 +440,7 @@ __device__ __forceinline__ void flush_tile(const E2hGemmParams& p, const __nv_bf
     if (t >= t_end || f >= p.F || in_tail(p, f)) continue;
     uint4 val = *reinterpret_cast<const uint4*>(tile + r * pitch + fv);
     __nv_bfloat16* dst = out + (long long)t * p.ldo + o_col + f;
-    if (p.epi == E2H_EPI_GATE) {
+    if (epi == E2H_EPI_GATE) {
       const uint4 gate = *reinterpret_cast<const uint4*>(dst);
       const __nv_bfloat162* g = reinterpret_cast<const __nv_bfloat162*>(&gate);
       __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&val);
@@ -439,7 +448,7 @@ __device__ __forceinline__ void flush_tile(const E2hGemmParams& p, const __nv_bf
       for (int k = 0; k < 4; ++k)
         o[k] = __floats2bfloat162_rn(__bfloat162float(o[k].x) * sigmoid_fast(__bfloat162float(g[k].x)),
                                      __bfloat162float(o[k].y) * sigmoid_fast(__bfloat162float(g[k].y)));
-    } else if (p.epi == E2H_EPI_RESIDUAL) {
+    } else if (epi == E2H_EPI_RESIDUAL) {
       const uint4 res = *reinterpret_cast<const uint4*>(
           static_cast<const __nv_bfloat16*>(p.aux) + (long long)t * p.ldo + f);
       const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&val);
@@ -451,15 +460,15 @@ __device__ __forceinline__ void flush_tile(const E2hGemmParams& p, const __nv_bf
         o[k] = __floats2bfloat162_rn(__bfloat162float(a[k].x) + __bfloat162float(b[k].x),
                                      __bfloat162float(a[k].y) + __bfloat162float(b[k].y));
       val = sum;
-    } else if (p.epi == E2H_EPI_ROPE_KV) {
+    } else if (epi == E2H_EPI_ROPE_KV) {
       const int D = p.head_dim;
       const int head = f / D;
       const int d = f - head * D;
       if (head >= p.n_head && p.kcache != nullptr) {
         const bool is_k = head < p.n_head + p.n_kv;
         const int hk = is_k ? head - p.n_head : head - p.n_head - p.n_kv;
-        const int b = t / p.sq;
-        const int pos = pos0 + (t - b * p.sq);
+        const int b = t / sq;
+        const int pos = pos0 + (t - b * sq);
         if (pos >= p.smax) continue;
         __nv_bfloat16* cache = static_cast<__nv_bfloat16*>(is_k ? p.kcache : p.vcache);
         dst = cache + (((long long)b * p.n_kv + hk) * p.smax + pos) * D + d;

@@ -71,14 +71,19 @@ struct SmemPlan {
   static constexpr int tmem_cols = acc_cols <= 32 ? 32 : acc_cols <= 64 ? 64 : acc_cols <= 128 ? 128 : acc_cols <= 256 ? 256 : 512;
 };
 
+// Epilogues that go through the staging tile where a launch has one compiled in.
+__host__ __device__ constexpr bool epi_stages(int epi) {
+  return epi != E2H_EPI_STORE_F32 && epi != E2H_EPI_RESIDUAL_F32;
+}
+
 // Exchange buffer for the cluster reduce: (S-1) sender slots x (BN/S) columns x 128 lanes fp32.
 __host__ __device__ inline int xchg_bytes(int bn, int splitk, int dual, int tf) {
   if (splitk <= 1) return 0;
   return (splitk - 1) * (bn / splitk) * tf * 4 * (dual ? 2 : 1);
 }
 
-template <int BN, bool DUAL, int TF>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int BN, bool DUAL, int TF, int EPI>
+__global__ void __launch_bounds__(kThreads, EPI >= 0 ? 2 : 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                  const __grid_constant__ CUtensorMap tmB, const E2hGemmParams p) {
   using Plan = SmemPlan<BN, DUAL, TF>;
@@ -170,8 +175,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // weight tiles (weights are never written by a preceding kernel of a PDL chain), the epilogue
   // warps wait before they touch the outputs, the MMA thread touches no global memory.
   pdl_launch_dependents();
-  const bool early_weights = kps > 1 && p.n_groups == 0;
-  if (!(warp == 0 && lane == 0 && early_weights) && !(warp == 1 && lane == 0)) pdl_wait_prior();
+  const bool early_weights = p.early != 0;
+  if (!(warp == 0 && lane == 0 && early_weights) && warp != 1) pdl_wait_prior();
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer ----------------
@@ -194,14 +199,24 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t a_dst = tiles0 + it * stage_sz;
         const int kb = kb_begin + it * kps;
         mbar_expect_tx(bar, kps * stage_bytes);
-        tma_load_3d_hint(a_dst, &tmA, 0, fa0, kb, bar, pol_a);
-        if (DUAL) tma_load_3d_hint(a_dst + kps * a_bytes, &tmA2, 0, fa0, kb, bar, pol_a);
+        if (kps > 1) {
+          tma_load_3d_hint(a_dst, &tmA, 0, fa0, kb, bar, pol_a);
+          if (DUAL) tma_load_3d_hint(a_dst + kps * a_bytes, &tmA2, 0, fa0, kb, bar, pol_a);
+        } else {
+          tma_load_2d_hint(a_dst, &tmA, kb * kTileK, fa0, bar, pol_a);
+          if (DUAL) tma_load_2d_hint(a_dst + a_bytes, &tmA2, kb * kTileK, fa0, bar, pol_a);
+        }
       }
       pdl_wait_prior();
       E2H_PHASE(p.phase_clock, 2);
-      for (int it = 0; it < n_pre; ++it)
-        tma_load_3d(tiles0 + it * stage_sz + kps * a_bytes * (DUAL ? 2 : 1), &tmB, 0, t0,
-                    kb_begin + it * kps, full0 + 8 * it);
+      for (int it = 0; it < n_pre; ++it) {
+        const uint32_t b_dst = tiles0 + it * stage_sz + kps * a_bytes * (DUAL ? 2 : 1);
+        const int kb = kb_begin + it * kps;
+        if (kps > 1)
+          tma_load_3d(b_dst, &tmB, 0, t0, kb, full0 + 8 * it);
+        else
+          tma_load_2d(b_dst, &tmB, b_col + kb * kTileK, t0, full0 + 8 * it);
+      }
       armed = n_pre;
       it0 = n_pre;
       s = n_pre == stages ? 0 : n_pre;
@@ -267,8 +282,12 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- UMMA issuer ----------------
+    // the whole warp walks the loop and one lane issues: the operands of an instruction are then
+    // uniform values, and it issues as fast as the tensor core takes it (M = 128, N = 64: 32 cycles;
+    // 50 to 66 from a branch of a single lane)
+    const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(TF, BN, p.a_mn_major, p.b_mn_major);
     const uint32_t a_kstep = p.a_mn_major ? 2048u : 32u;
     const uint32_t b_kstep = p.b_mn_major ? 2048u : 32u;
@@ -278,6 +297,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // descriptors: constant high word, base low words once, one add per instruction; stage and
     // phase are running counters (no division in this dependent scalar chain)
     const uint32_t d_hi = sw128_desc_hi(1024);
+    const uint32_t d0 = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t a_lo0 = sw128_desc_lo(smem_u32(tiles), a_lbo);
     const uint32_t b_lo0 = sw128_desc_lo(smem_u32(tiles), b_lbo);
     const uint32_t a_ks = a_kstep >> 4, b_ks = b_kstep >> 4;
@@ -285,16 +305,32 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t b_off = (kps * a_bytes * (DUAL ? 2 : 1)) >> 4;
     const uint32_t stage_step = (kps * stage_bytes) >> 4;
     const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
-    bool ok = true;
     int s = 0;
-    uint32_t ph = 0, st_lo = 0, accf = 0;
-    for (int it = 0; it < n_it && ok; ++it) {
-      ok = mbar_wait(full0 + 8 * s, ph, abort_flag, p.status, kStatusTimeoutFull);
-      if (!ok) break;
-      if (it == 0) E2H_PHASE(p.phase_clock, 4);
+    uint32_t ph = 0, st_lo = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const bool ok = mbar_wait(full0 + 8 * s, ph, abort_flag, p.status, kStatusTimeoutFull);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (it == 0 && lane == 0) E2H_PHASE(p.phase_clock, 4);
       tc_fence_after();
-      const uint32_t e_bar = empty0 + 8 * s;
-      const uint32_t cur_lo = st_lo;
+      // kps == 1: stage = [A][A2][B]; kps > 1: stage = [A x kps][A2 x kps][B x kps]
+      uint32_t a_lo = a_lo0 + st_lo, b_lo = b_lo0 + st_lo + b_off;
+      const int kcount = min(kps, n_kb - it * kps);
+      if (lead) {
+        for (int kk = 0; kk < kcount; ++kk) {
+#pragma unroll
+          for (int k = 0; k < kTileK / kUmmaK; ++k) {
+            const uint32_t accf = k > 0 || kk > 0 || it > 0;
+            umma_f16_lohi(d0, a_lo + k * a_ks, d_hi, b_lo + k * b_ks, d_hi, idesc, accf);
+            if (DUAL)
+              umma_f16_lohi(d0 + BN, a_lo + a2_off + k * a_ks, d_hi, b_lo + k * b_ks, d_hi, idesc,
+                            accf);
+          }
+          a_lo += a_bytes >> 4;
+          b_lo += Plan::b_bytes >> 4;
+        }
+        umma_commit(empty0 + 8 * s);  // stage reusable once these UMMAs have read it
+      }
+      __syncwarp();
       if (++s == stages) {
         s = 0;
         st_lo = 0;
@@ -302,25 +338,10 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else {
         st_lo += stage_step;
       }
-      const int kcount = min(kps, n_kb - it * kps);
-      // kps == 1: stage = [A][A2][B]; kps > 1: stage = [A x kps][A2 x kps][B x kps]
-      uint32_t a_lo = a_lo0 + cur_lo, b_lo = b_lo0 + cur_lo + b_off;
-      for (int kk = 0; kk < kcount; ++kk) {
-#pragma unroll
-        for (int k = 0; k < kTileK / kUmmaK; ++k) {
-          umma_f16_lohi(tmem_base, a_lo + k * a_ks, d_hi, b_lo + k * b_ks, d_hi, idesc, accf);
-          if (DUAL)
-            umma_f16_lohi(tmem_base + BN, a_lo + a2_off + k * a_ks, d_hi, b_lo + k * b_ks, d_hi,
-                          idesc, accf);
-          accf = 1;
-        }
-        a_lo += a_bytes >> 4;
-        b_lo += Plan::b_bytes >> 4;
-      }
-      umma_commit(e_bar);  // stage reusable once these UMMAs have read it
     }
-    umma_commit(smem_u32(&ctrl->tmem_full));
-    E2H_PHASE(p.phase_clock, 5);
+    if (lead) umma_commit(smem_u32(&ctrl->tmem_full));
+    __syncwarp();
+    if (lane == 0) E2H_PHASE(p.phase_clock, 5);
   }
 
   // ---------------- epilogue warps: accumulator -> registers ----------------
@@ -386,34 +407,34 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   // Staged epilogue: the finished values go through a [tokens][TH] bf16 tile in the (now idle)
   // pipeline buffers and leave with 16-byte accesses; see gemm_epilogue.cuh.
-  const bool staged = p.stage_epi != 0;
+  const int epi = EPI >= 0 ? EPI : p.epi;
+  const bool staged = EPI >= 0 ? epi_stages(EPI) : p.stage_epi != 0;
   __nv_bfloat16* stile = reinterpret_cast<__nv_bfloat16*>(tiles);
   if (is_epi && acc_ok) {
     const int c_begin = rank * slice;
     const int f = lane_valid ? f0 + lane_row : p.F;  // rows past F are masked in the epilogue
-    // columns of this warp: with 64 or more, alternate groups of 32; with fewer, the first /
-    // second half of the 8-column units
+    // columns of this warp: with 64 or more, alternate groups of W; with fewer, the first /
+    // second half of the 8-column units. W columns make one round trip to tensor memory (two
+    // accumulators of 32 would not fit the registers of two CTAs per SM)
+    constexpr int W = DUAL && EPI >= 0 ? 16 : 32;
     const int units = slice >> 3;
-    int c_first, c_last, c_step;
+    int c_first, c_last;
     if (units >= 8) {
-      c_first = 32 * half;
+      c_first = W * half;
       c_last = slice;
-      c_step = 64;
     } else {
       const int lo = units == 1 ? 1 : units >> 1;   // units of warp 0 (warp 1 takes the rest)
       c_first = half ? 8 * lo : 0;
       c_last = half ? slice : 8 * lo;
-      c_step = 64;
     }
     RopePre rope;
-    if (staged && p.epi == E2H_EPI_ROPE_KV) rope = rope_prepare(p, f);
-    for (int c = c_first; c < c_last; c += c_step) {
-      // up to 32 columns per round trip to tensor memory
-      const int nb = (c_last - c) >= 32 ? 4 : (c_last - c) / 8;
-      float v[32], v2[DUAL ? 32 : 1];
+    if (staged && epi == E2H_EPI_ROPE_KV) rope = rope_prepare(p, f);
+    for (int c = c_first; c < c_last; c += 2 * W) {
+      const int nb = (c_last - c) >= W ? W / 8 : (c_last - c) / 8;
+      float v[W], v2[DUAL ? W : 1];
       if (n_kb > 0) {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < W / 8; ++b) {
           if (b < nb) {
             issue_acc(0, c_begin + c + 8 * b, v + 8 * b);
             if constexpr (DUAL) issue_acc(1, c_begin + c + 8 * b, v2 + 8 * b);
@@ -422,13 +443,13 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_ld_wait();
       } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < W; ++j) {
           v[j] = 0.f;
           if constexpr (DUAL) v2[j] = 0.f;
         }
       }
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
+      for (int b = 0; b < W / 8; ++b) {
         if (b >= nb) continue;
         if (S > 1) {
           for (int slot = 0; slot < S - 1; ++slot) {
@@ -443,11 +464,11 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
         if (staged) {
-          stage8<DUAL>(p, f, t0 + c_begin + c + 8 * b, v + 8 * b, DUAL ? v2 + 8 * b : v2, stile,
-                       c + 8 * b, TH, lane_valid ? lane_row : -1, &rope, t_end);
+          stage8<DUAL, EPI>(p, f, t0 + c_begin + c + 8 * b, v + 8 * b, DUAL ? v2 + 8 * b : v2, stile,
+                            c + 8 * b, TH, lane_valid ? lane_row : -1, &rope, t_end);
         } else {
-          epilogue8<DUAL>(p, f, t0 + c_begin + c + 8 * b, v + 8 * b, DUAL ? v2 + 8 * b : v2,
-                            t_end, o_col);
+          epilogue8<DUAL, EPI>(p, f, t0 + c_begin + c + 8 * b, v + 8 * b, DUAL ? v2 + 8 * b : v2,
+                               t_end, o_col);
         }
       }
     }
@@ -456,7 +477,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (staged && is_epi) {
     asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps
     if (acc_ok)
-      flush_tile(p, stile, TH, f0, t0 + rank * slice, slice, threadIdx.x - 64, 256,
+      flush_tile<EPI>(p, stile, TH, f0, t0 + rank * slice, slice, threadIdx.x - 64, 256,
                  t_end, o_col);
   }
 
@@ -537,7 +558,7 @@ static int make_map3d(CUtensorMap* m, const void* base, long long K, long long r
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-template <int BN, bool DUAL, int TF>
+template <int BN, bool DUAL, int TF, int EPI>
 static int launch(const E2hGemmParams& p, const CUtensorMap& ta, const CUtensorMap& ta2,
                   const CUtensorMap& tb, cudaStream_t stream) {
   using Plan = SmemPlan<BN, DUAL, TF>;
@@ -546,7 +567,7 @@ static int launch(const E2hGemmParams& p, const CUtensorMap& ta, const CUtensorM
                       (size_t)p.stages * p.kps * (th * 128 * (DUAL ? 2 : 1) + Plan::b_bytes) +
                       xchg_bytes(BN, p.splitk, DUAL, TF);
   if (smem > 227 * 1024) return -12;
-  auto kern = umma_gemm_kernel<BN, DUAL, TF>;
+  auto kern = umma_gemm_kernel<BN, DUAL, TF, EPI>;
   static size_t configured = 0;  // per instantiation
   if (smem > configured) {
     cudaError_t e =
@@ -580,6 +601,19 @@ static int launch(const E2hGemmParams& p, const CUtensorMap& ta, const CUtensorM
   cfg.attrs = attrs;
   cfg.numAttrs = na;
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, ta2, tb, p);
+}
+
+// Whether a launch takes the kernels with the epilogue compiled in.
+static bool skinny_epi(const E2hGemmParams& p) {
+  if (p.tf != 128 || p.bn > 128 || p.a_mn_major || p.b_mn_major || p.a_tiled) return false;
+  if (p.n_groups == 0 && p.T > p.bn) return false;
+  if (p.n_groups > 0 && p.group_tmax > p.bn) return false;
+  if (p.dual ? p.epi != E2H_EPI_SWIGLU
+             : (p.epi == E2H_EPI_SWIGLU || p.epi == E2H_EPI_DUAL_STORE ||
+                p.epi == E2H_EPI_ROWMAJOR_F32_ACC || p.epi == E2H_EPI_ROWMAJOR_BF16))
+    return false;
+  if (p.epi == E2H_EPI_ROPE_KV && p.sq != 1) return false;
+  return !epi_stages(p.epi) || epi_can_stage(p, p.th);
 }
 
 }  // namespace e2h
@@ -621,8 +655,19 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   if (p.kps > 8) p.kps = 8;
   // several k-blocks per stage ride on 3-D boxes: K-major operands with K % 64 == 0 only
   if (p.a_mn_major || p.b_mn_major || p.a_tiled || p.n_batch > 0 || (p.K % 64) != 0) p.kps = 1;
-  const int stage_bytes = p.kps * (p.th * 128 * (p.dual ? 2 : 1) + p.bn * 128);
-  const int budget = 227 * 1024 - 2048 - xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
+  const int kb_bytes = p.th * 128 * (p.dual ? 2 : 1) + p.bn * 128;
+  // More CTAs than SMs: half the shared memory each, so that two share an SM, all of them run at
+  // once, and the next kernel of a PDL chain loads while the last ones finish (32016 x 4096, 64 rows:
+  // 57 -> 50 us; 2 x 22016 x 8192 gated: 169 -> 124). With fewer CTAs than SMs half a ring is too
+  // little in flight, and the next launch's CTAs crowd on the SMs that have both halves free
+  // (12288 x 4096 on 96 CTAs: 26 -> 32 us).
+  const bool skinny = skinny_epi(p);
+  const int ctas = ((p.F + p.th - 1) / p.th) * p.splitk *
+                   (p.n_groups > 0 ? p.n_groups : p.n_batch > 0 ? p.n_batch : 1);
+  const bool half = skinny && ctas > 148;
+  const int budget = (half ? 113 : 227) * 1024 - 2048 - xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
+  if (half) p.kps = 1;
+  const int stage_bytes = p.kps * kb_bytes;
   int max_stages = budget / stage_bytes;
   if (max_stages > kMaxStages) max_stages = kMaxStages;
   if (p.stages <= 0 || p.stages > max_stages) p.stages = max_stages;
@@ -674,24 +719,43 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   if (r) return r;
   }
 
-#define E2H_DISPATCH(BN_, DUAL_, TF_) return launch<BN_, DUAL_, TF_>(p, ta, ta2, tb, stream)
+  p.early = (p.kps > 1 || !(p.a_mn_major || p.b_mn_major || p.a_tiled)) && p.n_groups == 0;
+#define E2H_DISPATCH(BN_, DUAL_, TF_, EPI_) return launch<BN_, DUAL_, TF_, EPI_>(p, ta, ta2, tb, stream)
+#define E2H_SKINNY(EPI_)                                \
+  case EPI_:                                            \
+    if (p.bn == 64) E2H_DISPATCH(64, false, 128, EPI_); \
+    E2H_DISPATCH(128, false, 128, EPI_);
+  if (skinny && p.stage_epi == (epi_stages(p.epi) ? 1 : 0)) {
+    switch (p.epi) {
+      E2H_SKINNY(E2H_EPI_STORE_BF16)
+      E2H_SKINNY(E2H_EPI_STORE_F32)
+      E2H_SKINNY(E2H_EPI_RESIDUAL)
+      E2H_SKINNY(E2H_EPI_RESIDUAL_F32)
+      E2H_SKINNY(E2H_EPI_ROPE_KV)
+      E2H_SKINNY(E2H_EPI_GATE)
+      case E2H_EPI_SWIGLU:
+        if (p.bn == 64) E2H_DISPATCH(64, true, 128, E2H_EPI_SWIGLU);
+        E2H_DISPATCH(128, true, 128, E2H_EPI_SWIGLU);
+    }
+  }
+#undef E2H_SKINNY
   if (p.tf == 64) {
     if (p.dual) {
-      if (p.bn == 64) E2H_DISPATCH(64, true, 64);
-      E2H_DISPATCH(128, true, 64);
+      if (p.bn == 64) E2H_DISPATCH(64, true, 64, -1);
+      E2H_DISPATCH(128, true, 64, -1);
     } else {
-      if (p.bn == 64) E2H_DISPATCH(64, false, 64);
-      E2H_DISPATCH(128, false, 64);
+      if (p.bn == 64) E2H_DISPATCH(64, false, 64, -1);
+      E2H_DISPATCH(128, false, 64, -1);
     }
   }
   if (p.dual) {
-    if (p.bn == 64) E2H_DISPATCH(64, true, 128);
-    if (p.bn == 128) E2H_DISPATCH(128, true, 128);
-    E2H_DISPATCH(256, true, 128);
+    if (p.bn == 64) E2H_DISPATCH(64, true, 128, -1);
+    if (p.bn == 128) E2H_DISPATCH(128, true, 128, -1);
+    E2H_DISPATCH(256, true, 128, -1);
   } else {
-    if (p.bn == 64) E2H_DISPATCH(64, false, 128);
-    if (p.bn == 128) E2H_DISPATCH(128, false, 128);
-    E2H_DISPATCH(256, false, 128);
+    if (p.bn == 64) E2H_DISPATCH(64, false, 128, -1);
+    if (p.bn == 128) E2H_DISPATCH(128, false, 128, -1);
+    E2H_DISPATCH(256, false, 128, -1);
   }
 #undef E2H_DISPATCH
 }

@@ -89,6 +89,7 @@ struct E2hGemmParams {
   // matrix g multiplies the columns g * batch_k .. + K of every row of B and fills the columns
   // g * batch_out .. + F of every row of out
   int n_batch, batch_k, batch_out;
+  int early;             // set by e2h_gemm_umma: weights stream before the wait for the predecessor
 };
 
 #ifdef __cplusplus

@@ -61,8 +61,10 @@ def pick_tiles(F: int, T: int, K: int, dual: bool, splitk: Optional[int], bn: Op
     if splitk is None:
         splitk = 1
         if skinny:
-            while (splitk < 8 and tiles * splitk * 2 <= N_SM and kb // (splitk * 2) >= 4
-                   and bn % (splitk * 2 * 8) == 0):
+            # (clusters of eight that would take most of the SMs do not all find their places at
+            # once: 2048 x 2048 on 16 of them 14.0 us, on 16 clusters of four 7.7)
+            while (splitk < 8 and tiles * splitk * 2 <= (N_SM if splitk < 4 else 96)
+                   and kb // (splitk * 2) >= 4 and bn % (splitk * 2 * 8) == 0):
                 splitk *= 2
     if kps <= 0:
         if not skinny or K % 64:
@@ -83,22 +85,38 @@ class MulticastSignal:
         self.address = int(address)
 
 
-def pick_stream_tiles(F: int, K: int, bn: int, dual: bool):
-    """Feature-tile height of a skinny K-major GEMM that runs without split-K, or None to keep
-    128-row tiles. The kernel is a weight stream: with 128-row tiles a wide layer leaves SMs
-    idle (11008 features = 86 tiles on 148 SMs), with lower tiles one wave covers nearly all of
-    them (138 tiles of 80 rows). Measured on B200 at 64 tokens (cold L2): the dual w1/w3 GEMM
-    74 -> 54 us; single-accumulator GEMMs, whose tiles already cover 96+ SMs, and anything that
-    needs a split-K cluster (cluster placement, not the SM count, bounds its wave) do not gain,
-    so they keep their tiles."""
+def stream_plan(F: int, splitk: int, dual: bool):
+    """(feature-tile height, split-K) of a skinny K-major GEMM, or None to keep 128-row tiles. The
+    kernel is a weight stream: with 128-row tiles a wide layer leaves SMs idle, with lower tiles the
+    CTAs cover nearly all of them once, or twice at half the shared memory each (``e2h_gemm_umma``).
+    Measured on B200 at 64 tokens in a chain of launches (L2 cold):
+    gated 2 x 11008 x 4096, 86 tiles -> 138 of 80 rows: 74 -> 41 us; 2 x 22016 x 8192, 172 tiles in
+    two waves -> 276 resident ones of 80 rows: 169 -> 124; 12288 x 4096, 96 tiles -> 140 of 88 rows
+    with K in two: 25.1 -> 23.3, 10240 x 8192: 40.7 -> 36.3; 5120 x 5120, 40 tiles with K in two -> 72
+    of 72 rows with K in two: 16.8 -> 15.4; 32016 x 4096, 251 tiles -> 286 of 112 rows: 50.1 -> 48.9."""
+    def height(ctas):
+        th = max(64, -(-(-(-F // ctas)) // 8) * 8)
+        return th if th < 128 and -(-F // th) <= ctas else None
+
     tiles128 = -(-F // 128)
-    if tiles128 * 2 <= N_SM or tiles128 > N_SM or not dual:
+    if tiles128 > 2 * N_SM or (splitk > 1 and (dual or splitk != 2)):
         return None
-    th = -(-F // N_SM)
-    th = max(64, min(128, -(-th // 8) * 8))
-    if -(-F // th) > N_SM:
+    if tiles128 > N_SM:
+        th = height(2 * N_SM) if splitk == 1 else None
+        return th and (th, 1)
+    if splitk == 2:
+        th = height(N_SM // 2)
+        return th and (th, 2)
+    if tiles128 * 2 <= N_SM:
         return None
-    return th
+    th = height(N_SM)
+    return th and (th, 1 if dual else 2)
+
+
+def pick_stream_tiles(F: int, K: int, bn: int, dual: bool):
+    """Feature-tile height that ``stream_plan`` gives a GEMM whose K is not split beforehand."""
+    plan = stream_plan(F, 1, dual)
+    return plan and plan[0]
 
 
 ROWS_EPIS = {EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_RESIDUAL_F32, EPI_ROPE_KV}
@@ -227,10 +245,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
                   and K % 64 == 0 and STREAM_TILES)
     bn, splitk, stages, tf, kps = pick_tiles(F, T, K, dual, splitk, bn, stages, tf, kps)
     th = th or 0
-    if auto_tiles and not th and bn <= 128 and T <= bn and splitk == 1:
-        choice = pick_stream_tiles(F, K, bn, dual)
-        if choice is not None:
-            th, kps = choice, 4
+    if auto_tiles and not th and bn <= 128 and T <= bn:
+        choice = stream_plan(F, splitk, dual)
+        if choice is not None and -(-K // 64) // choice[1] >= 4:
+            th, splitk = choice
+            # k-blocks per stage: four, or two where four would leave a single stage
+            stage = _smem_bytes(bn, th, dual, splitk, 2, 4)
+            kps = 4 if stage <= 227 * 1024 else 2
     if (w8 or w4) and not th and splitk == 1 and STREAM_TILES:
         # the converting kernel is bound by bytes in flight per SM: a tile height that puts a
         # CTA on (nearly) every SM; rows per tile a multiple of 8 (int8) or 16 (int4)
