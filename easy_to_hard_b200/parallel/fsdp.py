@@ -47,6 +47,18 @@ def _group_size(group) -> Tuple[int, int]:
     return dist.get_world_size(group), dist.get_rank(group)
 
 
+def _as_dtype(x: torch.Tensor, dtype) -> torch.Tensor:
+    """``x.to(dtype)`` of a flat contiguous tensor; bf16 -> fp32 on the GPU in vector accesses (202M
+    gradients of a 7B layer: 535 -> 254 us)."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and dtype == torch.float32
+            and x.data_ptr() % 8 == 0):
+        return x.to(dtype)
+    from ..ops import _lib
+    out = torch.empty(x.shape, dtype=dtype, device=x.device)
+    _lib.check(_lib.lib().e2h_widen(x.data_ptr(), out.data_ptr(), x.numel(), _lib.stream()), "widen")
+    return out
+
+
 class ShardUnit:
     """One flat parameter: a list of (fqn, nn.Parameter) sharded over the data-parallel group."""
 
@@ -148,7 +160,7 @@ class ShardUnit:
                 dist.reduce_scatter_tensor(out, red, group=self.group)
             out = out.to(self.shard.dtype).div_(self.world)
         else:
-            out = full[: self.shard_size].to(self.shard.dtype)
+            out = _as_dtype(full[: self.shard_size], self.shard.dtype)
         if self.shard.grad is None:
             self.shard.grad = out.clone() if out.data_ptr() == full.data_ptr() else out
         else:

@@ -1,0 +1,75 @@
+"""The 16-byte forms of the optimizer, cast and cross-entropy kernels and the forms for rows that do not
+start on a 16-byte boundary, at the edges of both."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _adam64(p, g, m, v, kw):
+    p, g, m, v = (t.double() for t in (p, g, m, v))
+    p = p * (1 - kw["lr"] * kw["weight_decay"])
+    m = kw["beta1"] * m + (1 - kw["beta1"]) * g
+    v = kw["beta2"] * v + (1 - kw["beta2"]) * g * g
+    b1, b2 = 1 - kw["beta1"] ** kw["step"], 1 - kw["beta2"] ** kw["step"]
+    return p - kw["lr"] / b1 * m / ((v / b2).sqrt() + kw["eps"]), m, v
+
+
+@pytest.mark.parametrize("n", [1, 4, 1027, 500003])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("dts", [("f", "f", "f"), ("f", "b", "f"), ("b", "f", "b"), ("b", "b", "b")])
+def test_adamw(n, offset, dts):
+    """fp32: a dozen roundings of 2^-24; bf16 state and parameters: about eight of 2^-9."""
+    from easy_to_hard_b200.utils.memory_efficient_adam import fused_adamw_
+    dt = {"f": torch.float32, "b": torch.bfloat16}
+    g0 = torch.Generator(device="cuda").manual_seed(n)
+
+    def mk(kind, scale, positive=False):
+        t = torch.randn(n + offset, device="cuda", generator=g0) * scale
+        return (t.abs() + 1e-3 * scale if positive else t).to(dt[kind])[offset:]
+    p, g, m, v = mk(dts[0], 1.0), mk(dts[1], 1.0), mk(dts[2], 0.1), mk(dts[2], 0.1, True)
+    kw = dict(lr=0.01, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+    want = _adam64(p, g, m, v, kw)
+    copy = torch.zeros(n + offset, device="cuda", dtype=torch.bfloat16)[offset:]
+    fused_adamw_(p, g, m, v, bf16_copy=copy, **kw)
+    torch.cuda.synchronize()
+    for got, ref, kind in zip((p, m, v), want, (dts[0], dts[2], dts[2])):
+        tol = 2.0 ** -20 if kind == "f" and "b" not in dts else 2.0 ** -6
+        assert float((got.double() - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
+    assert torch.equal(copy, p.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (7, 4), (4099, 0), (1 << 20, 8), (33, 1)])
+def test_widening_is_exact(n, offset):
+    from easy_to_hard_b200.parallel.fsdp import _as_dtype
+    x = torch.randn(n + offset, device="cuda").bfloat16()[offset:]
+    assert torch.equal(_as_dtype(x, torch.float32), x.float())
+
+
+@pytest.mark.parametrize("vocab,pad", [(1, 3), (5, 0), (1000, 8), (8200, 1), (32016, 0)])
+def test_cross_entropy_rows(vocab, pad):
+    """fp32 sums of ``vocab`` terms and a few exponentials of 2 ulp: 1e-5; bf16 gradients: 2^-8."""
+    from easy_to_hard_b200.ops import loss
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = (torch.randn(6, vocab + pad, device="cuda", generator=g) * 5)[:, :vocab]
+    x[1] = -80.0
+    x[2, vocab // 2] = 60.0
+    t = torch.randint(0, vocab, (6,), device="cuda", generator=g)
+    z = x.double() / 0.7
+    lse = torch.logsumexp(z, -1)
+    p = torch.exp(z - lse[:, None])
+    st = loss.ce_stats(x, t, 0.7)
+    L, tgt, H = loss._combine_stats(st, None, 1)
+    assert float((L - lse).abs().max()) < 1e-5 * float(lse.abs().max().clamp_min(1))
+    assert float((tgt - z.gather(1, t[:, None])[:, 0]).abs().max()) < 1e-4
+    ent = lse - (p * z).sum(-1)
+    assert float((H - ent).abs().max()) < 1e-4 * float(lse.abs().max().clamp_min(1))
+    glp, gen = torch.randn(6, device="cuda"), torch.randn(6, device="cuda")
+    for ge in (None, gen):
+        d = loss.ce_grad(x, t, L, H, glp, ge, 0.7)
+        hot = torch.nn.functional.one_hot(t, vocab).double()
+        want = glp.double()[:, None] * (hot - p)
+        if ge is not None:
+            want = want - ge.double()[:, None] * p * (z - lse[:, None] + ent[:, None])
+        want = want / 0.7
+        assert float((d.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-4
