@@ -80,9 +80,91 @@ struct AttnWalk {
   int b, hk, ch, nc, start;
 };
 
+// Grouped heads (four or more query heads per kv head, head size 128) run on the tensor cores: see
+// attn_chunk_mma. Partial results of a CTA: one per half-warp, or one per warp there.
+template <int D, int G>
+struct AttnForm {
+  static constexpr bool mma = D == 128 && G >= 4 && G <= 8;
+  static constexpr int slots = mma ? kWarps : kSlots;
+};
+
+__device__ __forceinline__ void mma_16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// One chunk of 32 keys for the G <= 8 query heads of a kv head; warp w takes its keys 8 w .. 8 w + 7.
+// Lane (g, t): head g (rows 0..7 of the products), keys 2 t and 2 t + 1 of the warp's eight.
+//   scores: queries as A (rows), keys as B; the sum over the head's dims may run in any order, so both
+//     sides take 16 contiguous bytes per lane and 32 dims;
+//   output: the score fragment is the A fragment of the next product. The probabilities stay 32 bits
+//     wide: p = hi + mid + lo in bf16 (24 bits together), hi and mid side by side along the k
+//     dimension against the same values twice, lo in the unused rows 8..15.
+// On the CUDA cores every lane carried 8 heads x (8 queries + 8 sums) in registers and repeated the
+// softmax of its four keys 16 times over: 255 registers, one CTA of four warps per SM in two waves,
+// 113 us for 32 sequences x 8 kv heads x 724 keys (64 query heads); 33 now, the stream takes 14.
+template <int G>
+__device__ __forceinline__ void attn_chunk_mma(const uint8_t* ks, const uint8_t* vs, int warp, int lane,
+                                               int valid, float scale, const uint32_t (&qa)[4][4],
+                                               float& m, float& l, float (&o)[16][2]) {
+  const int g = lane >> 2, t = lane & 3;
+  float c[4] = {0.f, 0.f, 0.f, 0.f};
+  const uint8_t* krow = ks + (8 * warp + g) * 256 + t * 16;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    const uint4 kw = *reinterpret_cast<const uint4*>(krow + d * 64);
+    mma_16816(c, qa[d][0], 0u, qa[d][1], 0u, kw.x, kw.y);
+    mma_16816(c, qa[d][2], 0u, qa[d][3], 0u, kw.z, kw.w);
+  }
+  const int key = 8 * warp + 2 * t;
+  const bool ok0 = key < valid, ok1 = key + 1 < valid;
+  const float s0 = c[0] * scale, s1 = c[1] * scale;
+  float mn = m;
+  if (ok0) mn = fmaxf(mn, s0);
+  if (ok1) mn = fmaxf(mn, s1);
+  mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+  mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+  const float corr = __expf(m - mn);
+  const float p0 = ok0 ? __expf(s0 - mn) : 0.f, p1 = ok1 ? __expf(s1 - mn) : 0.f;
+  l = l * corr + (p0 + p1);
+  m = mn;
+  const float h0 = bf16_round(p0), h1 = bf16_round(p1);
+  const float r0 = p0 - h0, r1 = p1 - h1;
+  const float i0 = bf16_round(r0), i1 = bf16_round(r1);
+  const uint32_t hi = pack_bf16(h0, h1), mid = pack_bf16(i0, i1), lo = pack_bf16(r0 - i0, r1 - i1);
+  // rows that were not copied hold anything: their values must not meet a zero probability
+  const uint32_t keep = (ok0 ? 0x0000ffffu : 0u) | (ok1 ? 0xffff0000u : 0u);
+  const uint32_t vrow = smem_u32(vs) + (8 * warp + (lane & 7)) * 256 + (lane >> 3) * 16;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t v[4];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(vrow + j * 64)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t b = v[i] & keep;
+      float (&acc)[2] = o[4 * j + i];
+      float d[4] = {acc[0] * corr, acc[1] * corr, 0.f, 0.f};
+      mma_16816(d, hi, lo, mid, 0u, b, b);
+      acc[0] = d[0] + d[2];
+      acc[1] = d[1] + d[3];
+    }
+  }
+}
+
 // D = 16 * 8 * R : each lane of the half-warp holds R groups of 8 consecutive elements.
 template <int D, int G>
-__global__ void __launch_bounds__(kAttnThreads)
+__global__ void __launch_bounds__(kAttnThreads, AttnForm<D, G>::mma ? 3 : 0)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kcache,
                    const __nv_bfloat16* __restrict__ vcache, __nv_bfloat16* __restrict__ out,
                    float* __restrict__ partial, const int* __restrict__ pos_ptr,
@@ -106,8 +188,10 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   __shared__ int abort_word, nc_max_s, is_last_s;
   __shared__ int pre[kAttnMaxB + 1];     // chunks of the sequences before b (per kv head)
   __shared__ int first_key[kAttnMaxB];
-  __shared__ float sm_m[kSlots][G], sm_l[kSlots][G];
-  __shared__ float sm_acc[kSlots][G][D];
+  constexpr bool kMma = AttnForm<D, G>::mma;
+  constexpr int NS = AttnForm<D, G>::slots;
+  __shared__ float sm_m[NS][G], sm_l[NS][G];
+  __shared__ float sm_acc[NS][G][D];
   volatile int* abort_flag = &abort_word;
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -253,6 +337,51 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   for (int P = lo; P < hi;) {
     const int n_here = min(w.nc - w.ch, hi - P);
     const bool whole = w.ch == 0 && n_here == w.nc;
+    if constexpr (kMma) {
+      const int g = lane >> 2, t = lane & 3;
+      uint32_t qa[4][4];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+        if (g < G)
+          raw = *reinterpret_cast<const uint4*>(
+              q + ((long long)w.b * n_head + w.hk * G + g) * D + 32 * d + 8 * t);
+        qa[d][0] = raw.x;
+        qa[d][1] = raw.y;
+        qa[d][2] = raw.z;
+        qa[d][3] = raw.w;
+      }
+      float m = -FLT_MAX, l = 0.f, o[16][2];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = 0.f;
+      for (int c = 0; c < n_here; ++c) {
+        if (!dead && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag, status, kStatusTimeoutFull))
+          dead = true;
+        dead = __any_sync(0xffffffffu, dead);
+        if (!dead) {
+          const uint8_t* ks = attn_smem + s * 2 * kTileBytes;
+          attn_chunk_mma<G>(ks, ks + kTileBytes, warp, lane,
+                            pos + 1 - (w.start + (w.ch + c) * kChunk), scale, qa, m, l, o);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
+        }
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      if (g < G) {
+        if (t == 0) {
+          sm_m[warp][g] = m;
+          sm_l[warp][g] = l;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          *reinterpret_cast<float2*>(&sm_acc[warp][g][8 * i + 2 * t]) = make_float2(o[i][0], o[i][1]);
+      }
+    } else {
     float qv[G][R][8];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -377,6 +506,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
           for (int i = 0; i < 8; ++i) sm_acc[slot][g][(r * LPK + hl) * 8 + i] = acc[g][r][i];
       }
     }
+    }
     consumers_sync();
     // which of the pair's CTAs this one is, and how many there are
     int part, parts;
@@ -393,10 +523,10 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       const int g = idx / D, d = idx - g * D;
       float mm = -FLT_MAX;
 #pragma unroll
-      for (int t = 0; t < kSlots; ++t) mm = fmaxf(mm, sm_m[t][g]);
+      for (int t = 0; t < NS; ++t) mm = fmaxf(mm, sm_m[t][g]);
       float ll = 0.f, a = 0.f;
 #pragma unroll
-      for (int t = 0; t < kSlots; ++t) {
+      for (int t = 0; t < NS; ++t) {
         const float wt = (sm_m[t][g] == -FLT_MAX) ? 0.f : __expf(sm_m[t][g] - mm);
         ll += sm_l[t][g] * wt;
         a += sm_acc[t][g][d] * wt;
@@ -430,14 +560,26 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
           const int g = idx / D, d = idx - g * D;
           const int h = w.hk * G + g;
           const float* pp = partial + ((long long)w.b * n_head + h) * max_parts * (D + 2);
+          // all parts' loads before the first use: one round trip to L2 instead of three per part
+          float ms[kAttnMaxParts], ls[kAttnMaxParts], as[kAttnMaxParts];
+#pragma unroll
+          for (int t = 0; t < kAttnMaxParts; ++t) {
+            const float* pt = pp + (t < parts ? t : 0) * (D + 2);
+            ms[t] = __ldcg(pt + D);
+            ls[t] = __ldcg(pt + D + 1);
+            as[t] = __ldcg(pt + d);
+          }
           float mm = -FLT_MAX;
-          for (int t = 0; t < parts; ++t) mm = fmaxf(mm, __ldcg(pp + t * (D + 2) + D));
+#pragma unroll
+          for (int t = 0; t < kAttnMaxParts; ++t)
+            if (t < parts) mm = fmaxf(mm, ms[t]);
           float ll = 0.f, a = 0.f;
-          for (int t = 0; t < parts; ++t) {
-            const float ms = __ldcg(pp + t * (D + 2) + D);
-            const float wt = (ms == -FLT_MAX) ? 0.f : __expf(ms - mm);
-            ll += __ldcg(pp + t * (D + 2) + D + 1) * wt;
-            a += __ldcg(pp + t * (D + 2) + d) * wt;
+#pragma unroll
+          for (int t = 0; t < kAttnMaxParts; ++t) {
+            if (t >= parts) continue;
+            const float wt = (ms[t] == -FLT_MAX) ? 0.f : __expf(ms[t] - mm);
+            ll += ls[t] * wt;
+            a += as[t] * wt;
           }
           out[((long long)w.b * n_head + h) * D + d] =
               __float2bfloat16_rn(ll > 0.f ? a / ll : 0.f);
@@ -460,7 +602,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 // Resident CTAs per SM at this pipeline depth (shared memory is what limits them), at most 4.
 static int attn_ctas_per_sm(int D, int G, int stages) {
   // static shared memory of the kernel, plus the 1 KB that the system keeps per resident CTA
-  const int fixed = (2 * kAttnMaxB + 1) * 4 + kSlots * G * (D + 2) * 4 + 256 + 1024;
+  const int slots = D == 128 && G >= 4 && G <= 8 ? kWarps : kSlots;
+  const int fixed = (2 * kAttnMaxB + 1) * 4 + slots * G * (D + 2) * 4 + 256 + 1024;
   const int n = (227 * 1024) / (attn_smem_bytes(D, stages) + fixed);
   return n < 1 ? 1 : n > 4 ? 4 : n;
 }
