@@ -719,7 +719,10 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   if (r) return r;
   }
 
-  p.early = (p.kps > 1 || !(p.a_mn_major || p.b_mn_major || p.a_tiled)) && p.n_groups == 0;
+  // A holds weights, which no kernel of a PDL chain writes, except where the outputs are row-major: there
+  // the tokens lie on the lanes and A is what the predecessor may still be writing
+  p.early = !p.a_mn_major && !p.b_mn_major && !p.a_tiled && p.n_groups == 0 &&
+            p.epi != E2H_EPI_ROWMAJOR_F32_ACC && p.epi != E2H_EPI_ROWMAJOR_BF16;
 #define E2H_DISPATCH(BN_, DUAL_, TF_, EPI_) return launch<BN_, DUAL_, TF_, EPI_>(p, ta, ta2, tb, stream)
 #define E2H_SKINNY(EPI_)                                \
   case EPI_:                                            \

@@ -196,8 +196,7 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // ---------------- UMMA issuer ----------------
     // The whole warp walks the loop and one lane issues: the operands of an instruction are then
     // uniform values. In a branch of a single lane an instruction took 66 to 88 cycles to issue (64
-    // rows) where the tensor core takes 32, and the wait for the stage's own barrier another 220 per
-    // stage. 2 x 11008 x 4096 int8, 64 rows, one launch: 52.7 -> 48.2 us; 12288 x 4096: 32.1 -> 28.3.
+    // rows) where the tensor core takes 32. Chain of launches, 12288 x 4096 int8, 64 rows: 30.0 -> 27 us.
     // What is left is the converters' instruction issue.
     const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, BN, 0, 0);
@@ -206,16 +205,16 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const uint32_t d_hi = sw128_desc_hi(1024);
     const uint32_t d0 = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t b_lo0 = sw128_desc_lo(smem_u32(tiles) + AQ_BYTES * NMAT, 16);
-    const uint32_t empty0 = smem_u32(&ctrl->empty[0]);
+    const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
     const uint32_t cfull0 = smem_u32(&ctrl->conv_full[0]), cempty0 = smem_u32(&ctrl->conv_empty[0]);
     int s = 0, c = 0;
-    uint32_t cph = 0, st_lo = 0;
-    bool ok = true;
+    uint32_t cph = 0, ph = 0, st_lo = 0;
     for (int it = 0; it < n_it; ++it) {
-      // (the converters have seen the stage's full barrier before they arrive here)
-      ok = __all_sync(0xffffffffu, mbar_wait(cfull0 + 8 * c, cph, abort_flag, p.status,
-                                             kStatusTimeoutFull));
-      if (!ok) break;
+      // the converted tile first: the stage's own barrier (for the activation tile) has completed by then
+      const bool ok =
+          mbar_wait(cfull0 + 8 * c, cph, abort_flag, p.status, kStatusTimeoutFull) &&
+          mbar_wait(full0 + 8 * s, ph, abort_flag, p.status, kStatusTimeoutFull);
+      if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
       // A: 8 columns (16 k) per instruction, 32 columns per 64-wide k block
       const uint32_t a_col = d0 + kW8ACol0 + c * CONV_COLS, b_lo = b_lo0 + st_lo;
@@ -238,6 +237,7 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (++s == stages) {
         s = 0;
         st_lo = 0;
+        ph ^= 1;
       } else {
         st_lo += STAGE >> 4;
       }
