@@ -51,7 +51,7 @@ class GemmParams(C.Structure):
         ("n_groups", C.c_int), ("group_tmax", C.c_int), ("group_off", C.c_void_p),
         ("out_scale", C.c_float), ("softcap", C.c_float),
         ("n_batch", C.c_int), ("batch_k", C.c_int), ("batch_out", C.c_int),
-        ("early", C.c_int),
+        ("early", C.c_int), ("a_fresh", C.c_int),
     ]
 
 
@@ -147,6 +147,7 @@ _vp, _i, _ll, _f, _ull = C.c_void_p, C.c_int, C.c_longlong, C.c_float, C.c_ulong
 _SIGNATURES = {
     "e2h_gemm_umma": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_persistent": [C.POINTER(GemmParams), _vp],
+    "e2h_gemm_umma_plan": [C.POINTER(GemmParams), C.POINTER(C.c_int)],
     "e2h_gemm_w8": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_w4": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_f32": [C.POINTER(GemmParams), _vp],

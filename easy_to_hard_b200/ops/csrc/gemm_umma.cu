@@ -616,12 +616,9 @@ static bool skinny_epi(const E2hGemmParams& p) {
   return !epi_stages(p.epi) || epi_can_stage(p, p.th);
 }
 
-}  // namespace e2h
-
-extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
-  using namespace e2h;
-  E2hGemmParams p = *pp;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+// Checks the parameters and settles what a launch chooses by itself: tile height, k-blocks per
+// stage, stages, the form of the epilogue and whether weights are loaded early. 0 or an error code.
+static int umma_plan(E2hGemmParams& p) {
   if (p.F <= 0 || p.T <= 0 || p.K <= 0) return -1;
   if (p.bn != 64 && p.bn != 128 && p.bn != 256) return -2;
   if (p.splitk < 1 || p.splitk > 8 || (p.bn % (p.splitk * 8)) != 0) return -3;
@@ -642,8 +639,6 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   if ((p.out_scale != 0.f || p.softcap != 0.f) && p.epi != E2H_EPI_STORE_F32) return -5;
   if (p.epi == E2H_EPI_RESIDUAL_F32 && p.aux != p.out) return -5;
   if (p.tail_from && (p.epi != E2H_EPI_STORE_BF16 || p.tail == nullptr)) return -5;
-  const long long a_rows = (long long)p.F * (p.n_groups > 0 ? p.n_groups : p.n_batch > 0 ? p.n_batch : 1);
-  const long long b_cols = p.n_batch > 0 ? (long long)(p.n_batch - 1) * p.batch_k + p.K : p.K;
   if ((p.lda % 8) || (p.ldb % 8) || (p.dual && (p.lda2 % 8))) return -6;  // 16-byte strides for TMA
   if (((uintptr_t)p.a & 15) || ((uintptr_t)p.b & 15)) return -7;
   if (p.tf != 64 && p.tf != 128) p.tf = 128;
@@ -661,10 +656,9 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   // 57 -> 50 us; 2 x 22016 x 8192 gated: 169 -> 124). With fewer CTAs than SMs half a ring is too
   // little in flight, and the next launch's CTAs crowd on the SMs that have both halves free
   // (12288 x 4096 on 96 CTAs: 26 -> 32 us).
-  const bool skinny = skinny_epi(p);
   const int ctas = ((p.F + p.th - 1) / p.th) * p.splitk *
                    (p.n_groups > 0 ? p.n_groups : p.n_batch > 0 ? p.n_batch : 1);
-  const bool half = skinny && ctas > 148;
+  const bool half = skinny_epi(p) && ctas > 148;
   const int budget = (half ? 113 : 227) * 1024 - 2048 - xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
   if (half) p.kps = 1;
   const int stage_bytes = p.kps * kb_bytes;
@@ -682,6 +676,38 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   p.stage_epi = (epi_can_stage(p, p.th) &&
                  (long long)(p.bn / p.splitk) * p.th * 2 <= (long long)p.stages * stage_bytes)
                     ? 1 : 0;
+
+  // A holds weights, which no kernel of a PDL chain writes, except where the outputs are row-major (there
+  // the tokens lie on the lanes and A is what the predecessor may still be writing) and where the
+  // caller says that A is written in this stream
+  p.early = !p.a_mn_major && !p.b_mn_major && !p.a_tiled && p.n_groups == 0 && !p.a_fresh &&
+            p.epi != E2H_EPI_ROWMAJOR_F32_ACC && p.epi != E2H_EPI_ROWMAJOR_BF16;
+  return 0;
+}
+
+}  // namespace e2h
+
+// What e2h_gemm_umma would launch, without a GPU: out = {kps, stages, early, stage_epi}.
+extern "C" int e2h_gemm_umma_plan(const E2hGemmParams* pp, int* out) {
+  E2hGemmParams p = *pp;
+  const int r = e2h::umma_plan(p);
+  if (r) return r;
+  out[0] = p.kps;
+  out[1] = p.stages;
+  out[2] = p.early;
+  out[3] = p.stage_epi;
+  return 0;
+}
+
+extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
+  using namespace e2h;
+  E2hGemmParams p = *pp;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const int bad = umma_plan(p);
+  if (bad) return bad;
+  const int kb_total = (p.K + kTileK - 1) / kTileK;
+  const long long a_rows = (long long)p.F * (p.n_groups > 0 ? p.n_groups : p.n_batch > 0 ? p.n_batch : 1);
+  const long long b_cols = p.n_batch > 0 ? (long long)(p.n_batch - 1) * p.batch_k + p.K : p.K;
 
   CUtensorMap ta, ta2, tb;
   int r;
@@ -719,16 +745,12 @@ extern "C" int e2h_gemm_umma(const E2hGemmParams* pp, void* stream_v) {
   if (r) return r;
   }
 
-  // A holds weights, which no kernel of a PDL chain writes, except where the outputs are row-major: there
-  // the tokens lie on the lanes and A is what the predecessor may still be writing
-  p.early = !p.a_mn_major && !p.b_mn_major && !p.a_tiled && p.n_groups == 0 &&
-            p.epi != E2H_EPI_ROWMAJOR_F32_ACC && p.epi != E2H_EPI_ROWMAJOR_BF16;
 #define E2H_DISPATCH(BN_, DUAL_, TF_, EPI_) return launch<BN_, DUAL_, TF_, EPI_>(p, ta, ta2, tb, stream)
 #define E2H_SKINNY(EPI_)                                \
   case EPI_:                                            \
     if (p.bn == 64) E2H_DISPATCH(64, false, 128, EPI_); \
     E2H_DISPATCH(128, false, 128, EPI_);
-  if (skinny && p.stage_epi == (epi_stages(p.epi) ? 1 : 0)) {
+  if (skinny_epi(p) && p.stage_epi == (epi_stages(p.epi) ? 1 : 0)) {
     switch (p.epi) {
       E2H_SKINNY(E2H_EPI_STORE_BF16)
       E2H_SKINNY(E2H_EPI_STORE_F32)

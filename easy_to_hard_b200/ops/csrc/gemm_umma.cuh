@@ -90,6 +90,8 @@ struct E2hGemmParams {
   // g * batch_out .. + F of every row of out
   int n_batch, batch_k, batch_out;
   int early;             // set by e2h_gemm_umma: weights stream before the wait for the predecessor
+  int a_fresh;           // A (A2) is written by a kernel of the same stream, e.g. the bf16 image of a
+                         // quantised weight: never loaded before the wait
 };
 
 #ifdef __cplusplus

@@ -173,6 +173,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
     matrix first for larger token counts."""
     assert a.is_cuda and b.is_cuda and b.dtype == torch.bfloat16
     w4 = isinstance(a, Int4Weight)
+    fresh = False           # whether a is written by a launch of this call
     rows = (not (a_mn_major or b_mn_major or n_groups or signal or stages) and tiled_shape is None
             and batch is None and splitk is None and bn is None and tf is None and th is None
             and kps <= 0 and persistent is None and pair is None and rows_rule(a, a2, b, epi))
@@ -184,7 +185,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
                          or (K4 // 2) % 16):
             a = _expand_int4(a, 0)            # many tokens: one dequantisation pass, then bf16
             a2 = _expand_int4(a2, 1) if a2 is not None else None
-            w4 = False
+            w4, fresh = False, True
     w8 = not w4 and a.dtype == torch.int8
     if w8:
         assert scale is not None and not a_mn_major and not b_mn_major and tiled_shape is None
@@ -193,7 +194,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         if not rows and (b.shape[0] > 128 or a.shape[1] % 128 or _ld(a) % 16):
             a = _expand_int8(a, 0)
             a2 = _expand_int8(a2, 1) if a2 is not None else None
-            w8 = False
+            w8, fresh = False, True
     assert w8 or w4 or a.dtype == torch.bfloat16
     if w4:
         F, K = a.shape
@@ -280,6 +281,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
             p.signal[i] = f if isinstance(f, int) else f.data_ptr()
         p.ticket = ticket.data_ptr()
     p.kps = kps
+    p.a_fresh = int(fresh)
     p.a_tiled = int(tiled_shape is not None)
     if w4:
         p.lda, p.ldb = _ld(a.q), _ld(b)

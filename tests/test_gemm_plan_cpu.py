@@ -1,0 +1,80 @@
+"""What a GEMM call hands to the tcgen05 kernel for one token tile (csrc/gemm_umma.cu) and what the
+kernel's host side makes of it, without a GPU: the launch is recorded instead of made."""
+import ctypes as C
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from easy_to_hard_b200.ops import _lib, gemm
+
+
+class OnGpu:
+    """A CPU tensor that says it is a CUDA one."""
+    is_cuda = True
+
+    def __init__(self, t):
+        self._t = t
+
+    def __getattr__(self, name):
+        return getattr(self._t, name)
+
+
+def _plan(p):
+    """(k-blocks per stage, stages, loads weights early, staged epilogue) of a launch."""
+    out = (C.c_int * 4)()
+    rc = _lib.lib().e2h_gemm_umma_plan(C.byref(p), out)
+    return rc if rc else tuple(out)
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """The parameter blocks of the e2h_gemm_umma launches of a test."""
+    seen = []
+
+    def record(ref, stream):
+        p = _lib.GemmParams()
+        C.memmove(C.byref(p), ref, C.sizeof(p))
+        seen.append(p)
+        return 0
+    _lib.lib()
+    word = torch.zeros(1, dtype=torch.int32)
+    fake = SimpleNamespace(e2h_gemm_umma=record)
+    monkeypatch.setattr(gemm, "_lib", SimpleNamespace(
+        lib=lambda: fake, stream=lambda: 0, check=_lib.check, status_word=lambda device: word))
+    monkeypatch.setattr(gemm, "_expand_int8", lambda w, which: OnGpu(w._t.to(torch.bfloat16)))
+    monkeypatch.setattr(gemm, "_expand_int4", lambda w, which: OnGpu(w.dequant()))
+    return seen
+
+
+# (whole int8 / int4 tiles of up to 128 tokens stream through a kernel of their own, gated products of
+# more tokens through another)
+CASES = [(bits, T, K, dual) for bits in (16, 8, 4) for T in (17, 64, 128, 200)
+         for K in (688, 1024, 1376) for dual in (False, True)
+         if not (bits != 16 and T <= 128 and K % 128 == 0) and not (dual and T > 128)]
+
+
+@pytest.mark.parametrize("bits,T,K,dual", CASES)
+def test_weights_expanded_by_the_call_are_not_loaded_early(launches, bits, T, K, dual):
+    """The bf16 image of a quantised matrix is written by the launch before: loads ahead of the wait for
+    that launch could read what the buffer held before."""
+    F = 256
+    x = OnGpu(torch.zeros(T, K, dtype=torch.bfloat16))
+
+    def weight():
+        if bits == 16:
+            return OnGpu(torch.zeros(F, K, dtype=torch.bfloat16))
+        if bits == 8:
+            return OnGpu(torch.zeros(F, K, dtype=torch.int8))
+        g = 16 if K == 688 else 32
+        w = gemm.Int4Weight.from_int(torch.zeros(F, K, dtype=torch.int32), torch.zeros(K // g, F, 2), g)
+        w.is_cuda = True
+        return w
+    out = OnGpu(torch.zeros(T, F, dtype=torch.bfloat16))
+    scale = OnGpu(torch.zeros((1 + dual) * F)) if bits == 8 else None
+    if dual:
+        gemm.linear_swiglu(x, weight(), weight(), out=out, scale=scale)
+    else:
+        gemm.linear(x, weight(), out=out, scale=scale)
+    assert len(launches) == 1
+    assert _plan(launches[0])[2] == (bits == 16)
