@@ -169,8 +169,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
     multiplied by matrix g (at most ``group_tmax`` rows each). Shapes: a is [F, K] (or [K, F] when
     a_mn_major), b is [T, K] (or [K, T]).
     An int8 ``a`` (weight-only quantisation; ``scale`` holds the per-feature scales) streams as
-    int8 through the converting kernel for up to 128 tokens and is expanded to a scratch bf16
-    matrix first for larger token counts."""
+    int8 through the converting kernel for up to 128 tokens and is expanded to a bf16 matrix first
+    for larger token counts."""
     assert a.is_cuda and b.is_cuda and b.dtype == torch.bfloat16
     w4 = isinstance(a, Int4Weight)
     fresh = False           # whether a is written by a launch of this call
@@ -408,7 +408,6 @@ class Int4Weight:
         return (x * s + z).view(F, K)
 
 
-_INT8_SCRATCH: dict = {}
 # large GEMMs on CTA pairs (cta_group::2, 256 x 256 tiles): E2H_GEMM_PAIR=0 keeps single-CTA tiles
 PAIR_DEFAULT = os.environ.get("E2H_GEMM_PAIR", "1") != "0"
 # skinny GEMMs: feature-tile height and split-K chosen so that the tiles fill one wave of the SMs
@@ -417,15 +416,12 @@ STREAM_TILES = os.environ.get("E2H_STREAM_TILES", "1") != "0"
 
 
 def _expand_int8(w: torch.Tensor, which: int) -> torch.Tensor:
-    """bf16 image of an int8 weight in a per-device scratch buffer (two buffers, so that both
-    matrices of a dual GEMM can be live). Used for token counts where re-converting the weights
-    per token tile would cost more than one expansion pass."""
-    key = (w.device.index, which)
-    buf = _INT8_SCRATCH.get(key)
-    if buf is None or buf.numel() < w.numel():
-        buf = torch.empty(w.numel(), dtype=torch.bfloat16, device=w.device)
-        _INT8_SCRATCH[key] = buf
-    out = buf[: w.numel()].view(w.shape)
+    """bf16 image of an int8 weight (``which``: 0, or 1 for the second matrix of a gated product). Used
+    for token counts where re-converting the weights per token tile would cost more than one
+    expansion pass. Every image has memory of its own from the caching allocator, which orders its
+    reuse by stream and keeps it with the graph if the call is captured: a buffer kept here could be
+    replaced by a larger one under a captured step, or shared by two streams."""
+    out = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
     F, K = w.shape
     if K % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 8 == 0:
         _lib.check(_lib.lib().e2h_expand_weight(w.data_ptr(), w.stride(0), 8, None, 0, out.data_ptr(),
@@ -436,14 +432,8 @@ def _expand_int8(w: torch.Tensor, which: int) -> torch.Tensor:
 
 
 def _expand_int4(w: "Int4Weight", which: int) -> torch.Tensor:
-    """bf16 image of an int4 weight in the per-device scratch buffers of ``_expand_int8``."""
-    key = (w.device.index, which)
-    n = w.shape[0] * w.shape[1]
-    buf = _INT8_SCRATCH.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.empty(n, dtype=torch.bfloat16, device=w.device)
-        _INT8_SCRATCH[key] = buf
-    out = buf[:n].view(w.shape)
+    """bf16 image of an int4 weight, as ``_expand_int8``."""
+    out = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
     F, K = w.shape
     if w.groupsize % 8 == 0 and w.q.stride(1) == 1 and w.q.stride(0) % 4 == 0:
         _lib.check(_lib.lib().e2h_expand_weight(w.q.data_ptr(), w.q.stride(0), 4, w.sz.data_ptr(),

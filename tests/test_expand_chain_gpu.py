@@ -66,3 +66,47 @@ def test_products_alternate_through_the_expansion(bits, T, K):
         for (_, _, wf), out in zip(ws, outs):
             _close(out, x.double() @ wf.double().t(), x, wf)
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+def test_a_captured_step_keeps_its_image(bits):
+    """A larger matrix is expanded after the capture, and memory that comes free is taken and filled:
+    the step still gives its product, and writes into nothing else."""
+    from easy_to_hard_b200.ops import _lib, gemm
+    T, K = 160, 1024
+    w, s, wf = _weight(512, K, bits, 1)
+    x = torch.randn(T, K, device="cuda").bfloat16()
+    out = torch.empty(T, 512, device="cuda", dtype=torch.bfloat16)
+    g = _captured(lambda: gemm.linear(x, w, out=out, scale=s))
+    big, sb, bf = _weight(9000, K, bits, 2)
+    got = gemm.linear(x, big, scale=sb)
+    _close(got, x.double() @ bf.double().t(), x, bf)
+    torch.cuda.synchronize()
+    taken = [torch.full((n * K,), 7.0, device="cuda", dtype=torch.bfloat16)
+             for n in (512, 512, 512, 9000)]
+    x.copy_(torch.randn(T, K, device="cuda"))
+    g.replay()
+    torch.cuda.synchronize()
+    _close(out, x.double() @ wf.double().t(), x, wf)
+    assert all(bool((t == 7.0).all()) for t in taken)
+    assert _lib.read_status() == 0
+
+
+def test_two_streams_expand_at_once():
+    from easy_to_hard_b200.ops import _lib, gemm
+    T, K = 160, 2048
+    ws = [_weight(8192, K, 8, n) for n in (3, 4)]
+    x = torch.randn(T, K, device="cuda").bfloat16()
+    want = [x.double() @ wf.double().t() for _, _, wf in ws]
+    streams = [torch.cuda.Stream() for _ in ws]
+    outs = [torch.empty(20, T, 8192, device="cuda", dtype=torch.bfloat16) for _ in ws]
+    torch.cuda.synchronize()
+    for i in range(20):
+        for (w, s, _), st, out in zip(ws, streams, outs):
+            with torch.cuda.stream(st):
+                gemm.linear(x, w, out=out[i], scale=s)
+    torch.cuda.synchronize()
+    for (_, _, wf), out, ref in zip(ws, outs, want):
+        for i in range(20):
+            _close(out[i], ref, x, wf)
+    assert _lib.read_status() == 0

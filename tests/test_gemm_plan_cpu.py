@@ -78,3 +78,16 @@ def test_weights_expanded_by_the_call_are_not_loaded_early(launches, bits, T, K,
         gemm.linear(x, weight(), out=out, scale=scale)
     assert len(launches) == 1
     assert _plan(launches[0])[2] == (bits == 16)
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_the_image_of_a_matrix_is_not_overwritten_by_the_next(which):
+    """A captured step keeps the address of its image, another stream may still read it."""
+    small, large = (torch.randint(-128, 128, (n, 12), dtype=torch.int8) for n in (5, 40))
+    images = [(w, gemm._expand_int8(w, which)) for w in (small, large, small + 1, small)]
+    codes = torch.randint(0, 16, (6, 8), dtype=torch.int32)
+    w4 = gemm.Int4Weight.from_int(codes, torch.rand(2, 6, 2), 4)
+    images.append((w4.dequant(), gemm._expand_int4(w4, which)))
+    for w, image in images:
+        assert torch.equal(image, w.to(torch.bfloat16))
+    assert len({image.untyped_storage().data_ptr() for _, image in images}) == len(images)
