@@ -146,6 +146,18 @@ def rope(x: torch.Tensor, freqs: torch.Tensor, pos: torch.Tensor, n_heads: int, 
 _ATTN_SCRATCH: dict = {}
 
 
+def _attn_scratch(device, floats: int, words: int):
+    """(partial results, zeroed ticket words) for decode attention on one device. A captured step keeps
+    their addresses, so that a buffer that has become too small stays alive beside the larger one; every
+    new one is at least twice the one before, the kept ones together are no more than the last."""
+    kept = _ATTN_SCRATCH.setdefault(device.index, [])
+    if not kept or kept[-1][0].numel() < floats or kept[-1][1].numel() < words:
+        old = [t.numel() for t in kept[-1]] if kept else [1 << 19, 2048]
+        kept.append((torch.empty(max(floats, 2 * old[0]), dtype=torch.float32, device=device),
+                     torch.zeros(max(words, 2 * old[1]), dtype=torch.int32, device=device)))
+    return kept[-1]
+
+
 def attn_decode_splits(B: int, n_kv: int, smax: Optional[int] = None) -> int:
     """How many CTAs may share one (sequence, kv head) in ``attn_decode``: the kernel deals the
     32-key chunks of all pairs out evenly, so a pair may be cut by run boundaries; 8 lets the
@@ -175,15 +187,9 @@ def attn_decode(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, pos
     tickets = None
     if n_split > 1:
         need = B * n_head * n_split * (D + 2)
-        key = q.device.index
-        buf = _ATTN_SCRATCH.get(key)
-        if buf is None or buf[0].numel() < need or buf[1].numel() < B * n_kv:
-            buf = (torch.empty(max(need, 1 << 20), dtype=torch.float32, device=q.device),
-                   torch.zeros(max(B * n_kv, 4096), dtype=torch.int32, device=q.device))
-            _ATTN_SCRATCH[key] = buf
-        tickets = buf[1]
+        buf, tickets = _attn_scratch(q.device, need, B * n_kv)
         if scratch is None:
-            scratch = buf[0]
+            scratch = buf
         assert scratch.numel() >= need and scratch.dtype == torch.float32
     rc = _lib.lib().e2h_attn_decode(q.data_ptr(), kcache.data_ptr(), vcache.data_ptr(),
                                     out.data_ptr(), _lib.ptr(scratch), pos.data_ptr(),

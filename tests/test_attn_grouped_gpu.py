@@ -31,3 +31,32 @@ def test_against_64_bits(G, pos, pad, n_split):
     want = (torch.softmax(s, -1)[..., None] * v).sum(2)
     err = (out.double().view(B, n_kv * G, D) - want).abs()
     assert bool((err <= 2.0 ** -8 * want.abs() + 2.0 ** -17 * v.abs().max()).all())
+
+
+def test_a_captured_step_survives_a_larger_batch():
+    """The scratch of a captured launch stays its own when a larger batch asks for more."""
+    from easy_to_hard_b200.ops import _lib, functional as Fn
+    n_kv, G, D, smax = 8, 8, 128, 512
+    at = torch.tensor([500], dtype=torch.int32, device="cuda")
+
+    def case(B):
+        g = torch.Generator(device="cuda").manual_seed(B)
+        return (torch.randn(B, n_kv * G * D, device="cuda", generator=g).bfloat16(),
+                *(torch.randn(B, n_kv, smax, D, device="cuda", generator=g).bfloat16()
+                  for _ in range(2)))
+    small = case(2)
+    want = Fn.attn_decode(*small, at, None, n_kv * G)
+    out = torch.empty_like(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        Fn.attn_decode(*small, at, None, n_kv * G, out=out)
+    Fn.attn_decode(*case(96), at, None, n_kv * G)
+    torch.cuda.synchronize()
+    taken = [torch.full((n,), -1, device="cuda", dtype=torch.int32) for n in (1 << 20, 4096, 4096)]
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert all(bool((t == -1).all()) for t in taken)
+    assert _lib.read_status() == 0

@@ -95,3 +95,25 @@ def test_every_chunk_once_and_parts_fit(seed):
         assert 2 <= parts <= max(max_parts, 2), key
     if max_parts <= 1:
         assert not parts_of
+
+
+def test_scratch_outlives_a_larger_batch(monkeypatch):
+    """A captured step keeps the address of its scratch: the buffers are never dropped, and the kept ones
+    stay below the last one together."""
+    import gc
+    import weakref
+
+    import torch
+
+    from easy_to_hard_b200.ops import functional as Fn
+    monkeypatch.setattr(Fn, "_ATTN_SCRATCH", {})
+    cpu, seen = torch.device("cpu"), []
+    for floats, words in ((1000, 8), (1 << 20, 64), (1 << 21, 64), (3, 5000), ((1 << 22) + 5, 64)):
+        part, tickets = Fn._attn_scratch(cpu, floats, words)
+        assert part.numel() >= floats and tickets.numel() >= words and not tickets.any()
+        if part.data_ptr() not in {p for p, _, _ in seen}:
+            seen.append((part.data_ptr(), part.numel(), weakref.ref(part)))
+    del part, tickets
+    gc.collect()
+    assert all(ref() is not None for _, _, ref in seen) and len(seen) > 2
+    assert sum(n for _, n, _ in seen[:-1]) <= seen[-1][1]
