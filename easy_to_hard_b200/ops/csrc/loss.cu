@@ -28,6 +28,12 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
   return t;
 }
 
+// A sum moved to a higher maximum. Where the factor is 0 the sum is left out: entries at the lowest finite
+// value (a mask) make u infinite, and 0 * -inf would be NaN. A NaN stays.
+__device__ __forceinline__ float ce_rescale(float v, float r) {
+  return r == 0.f && !isnan(v) ? 0.f : v * r;
+}
+
 // Running (max, sum of exp, sum of exp * z) of N more values.
 template <int N>
 __device__ __forceinline__ void ce_step(const float* z, float& m, float& s, float& u) {
@@ -36,8 +42,8 @@ __device__ __forceinline__ void ce_step(const float* z, float& m, float& s, floa
   for (int k = 0; k < N; ++k) mn = fmaxf(mn, z[k]);
   if (mn > m) {
     const float r = __expf(m - mn);
-    s *= r;
-    u *= r;
+    s = ce_rescale(s, r);
+    u = ce_rescale(u, r);
     m = mn;
   }
 #pragma unroll
@@ -96,8 +102,8 @@ ce_stats_kernel(const float* __restrict__ logits, long long ld, int vocab,
   }
   const float gm = block_reduce(m, red, true);
   const float r = __expf(m - gm);       // (a thread without values: s = u = 0)
-  s = block_reduce(s * r, red, false);
-  u = block_reduce(u * r, red, false);
+  s = block_reduce(ce_rescale(s, r), red, false);
+  u = block_reduce(ce_rescale(u, r), red, false);
   if (threadIdx.x == 0) {
     const long long t = targets[row] - vocab_start;
     const float tgt = (t >= 0 && t < vocab) ? x[t] * inv_temp : 0.f;
@@ -161,9 +167,9 @@ extern "C" int e2h_ce_stats(const float* logits, long long ld, int rows, int voc
                             float* stats, void* stream) {
   using namespace e2h;
   const bool vec = ((uintptr_t)logits & 15) == 0 && ld % 4 == 0;
-  return (int)launch(vec ? ce_stats_kernel<true> : ce_stats_kernel<false>, dim3(rows), dim3(kCeThreads), 0, (cudaStream_t)stream,
-                     logits, ld, vocab, targets, vocab_start, inv_temp,
-                     reinterpret_cast<float4*>(stats));
+  return (int)launch(vec ? ce_stats_kernel<true> : ce_stats_kernel<false>, dim3(rows),
+                     dim3(kCeThreads), 0, (cudaStream_t)stream, logits, ld, vocab, targets,
+                     vocab_start, inv_temp, reinterpret_cast<float4*>(stats));
 }
 
 extern "C" int e2h_ce_grad(const float* logits, long long ld, int rows, int vocab,
@@ -172,7 +178,8 @@ extern "C" int e2h_ce_grad(const float* logits, long long ld, int rows, int voca
                            const float* g_ent, void* dlogits, long long ldd, void* stream) {
   using namespace e2h;
   const bool vec = (((uintptr_t)logits | (uintptr_t)dlogits) & 15) == 0 && ld % 4 == 0 && ldd % 8 == 0;
-  return (int)launch(vec ? ce_grad_kernel<true> : ce_grad_kernel<false>, dim3(rows), dim3(kCeThreads), 0, (cudaStream_t)stream,
-                     logits, ld, vocab, targets, vocab_start, inv_temp, lse, ent, g_lp, g_ent,
+  return (int)launch(vec ? ce_grad_kernel<true> : ce_grad_kernel<false>, dim3(rows),
+                     dim3(kCeThreads), 0, (cudaStream_t)stream, logits, ld, vocab, targets,
+                     vocab_start, inv_temp, lse, ent, g_lp, g_ent,
                      static_cast<__nv_bfloat16*>(dlogits), ldd);
 }

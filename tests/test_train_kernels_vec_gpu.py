@@ -73,3 +73,38 @@ def test_cross_entropy_rows(vocab, pad):
             want = want - ge.double()[:, None] * p * (z - lse[:, None] + ent[:, None])
         want = want / 0.7
         assert float((d.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-4
+
+
+@pytest.mark.parametrize("vocab,pad", [(5, 0), (1000, 8), (4096, 0), (8200, 1), (32016, 0)])
+def test_cross_entropy_of_masked_rows(vocab, pad):
+    """Entries at the lowest finite value add nothing, wherever they lie and however many threads meet
+    nothing else; a NaN or an infinite entry still shows. Bounds as above."""
+    from easy_to_hard_b200.ops import loss
+    low = torch.finfo(torch.float32).min
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = (torch.randn(7, vocab + pad, device="cuda", generator=g) * 5)[:, :vocab]
+    drop = torch.rand(7, vocab, device="cuda", generator=g)
+    x[0, drop[0] < 0.75] = low
+    x[1, : vocab - 1] = low
+    x[2, 1:] = low
+    x[3, ::2] = low
+    x[4, : vocab // 2] = low
+    x[5] = low
+    x[5, vocab // 3] = -1e30
+    x[:, vocab // 2] = torch.where(x[:, vocab // 2] == low, x[:, vocab // 2], 3.0)
+    t = torch.full((7,), vocab // 2, device="cuda")
+    z = x.double()
+    lse = torch.logsumexp(z, -1)
+    p = torch.exp(z - lse[:, None])
+    L, tgt, H = loss._combine_stats(loss.ce_stats(x, t), None, 1)
+    scale = lse.abs().clamp_min(1)
+    assert float(((L - lse).abs() / scale).max()) < 1e-5
+    ent = -(p * torch.where(p > 0, z - lse[:, None], 0.0)).sum(-1)
+    assert float(((H - ent).abs() / scale).max()) < 1e-4
+    d = loss.ce_grad(x, t, L, H, torch.ones(7, device="cuda"), torch.ones(7, device="cuda"))
+    assert bool(torch.isfinite(d).all())
+    for bad in (float("nan"), float("inf")):
+        y = x.clone()
+        y[:, 0], y[:, -1] = bad, 500.0
+        L, _, H = loss._combine_stats(loss.ce_stats(y, t), None, 1)
+        assert bool(torch.isnan(L).all()) and bool(torch.isnan(H).all())
