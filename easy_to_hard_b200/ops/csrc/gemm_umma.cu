@@ -26,6 +26,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <math.h>
 #include <stdio.h>
 #include <string.h>
 #include <mutex>
@@ -616,6 +617,15 @@ static bool skinny_epi(const E2hGemmParams& p) {
   return !epi_stages(p.epi) || epi_can_stage(p, p.th);
 }
 
+// How many groups of a grouped product will have rows, as far as the host can tell: T rows are at most
+// group_tmax tokens with T / group_tmax different groups each.
+static int live_groups(const E2hGemmParams& p) {
+  const int tokens = p.group_tmax < p.T ? p.group_tmax : p.T;
+  const double share = (double)p.T / ((double)tokens * p.n_groups);
+  const double live = share >= 1.0 ? p.n_groups : p.n_groups * (1.0 - pow(1.0 - share, tokens));
+  return (int)(live + 0.5);
+}
+
 // Checks the parameters and settles what a launch chooses by itself: tile height, k-blocks per
 // stage, stages, the form of the epilogue and whether weights are loaded early. 0 or an error code.
 static int umma_plan(E2hGemmParams& p) {
@@ -655,11 +665,14 @@ static int umma_plan(E2hGemmParams& p) {
   // once, and the next kernel of a PDL chain loads while the last ones finish (32016 x 4096, 64 rows:
   // 57 -> 50 us; 2 x 22016 x 8192 gated: 169 -> 124). With fewer CTAs than SMs half a ring is too
   // little in flight, and the next launch's CTAs crowd on the SMs that have both halves free
-  // (12288 x 4096 on 96 CTAs: 26 -> 32 us).
+  // (12288 x 4096 on 96 CTAs: 26 -> 32 us). What counts is CTAs with work: of 8 experts, 2 x 2752 x 2048
+  // gated, with two live ones 20.7 us at the full ring, 33.4 at half; with all eight 61 and 45. Half a
+  // ring of one stage would not overlap loads and products: it takes two beside the exchange buffer.
+  const int xchg = xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
   const int ctas = ((p.F + p.th - 1) / p.th) * p.splitk *
-                   (p.n_groups > 0 ? p.n_groups : p.n_batch > 0 ? p.n_batch : 1);
-  const bool half = skinny_epi(p) && ctas > 148;
-  const int budget = (half ? 113 : 227) * 1024 - 2048 - xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
+                   (p.n_groups > 0 ? live_groups(p) : p.n_batch > 0 ? p.n_batch : 1);
+  const bool half = skinny_epi(p) && ctas > 148 && 113 * 1024 - 2048 - xchg >= 2 * kb_bytes;
+  const int budget = (half ? 113 : 227) * 1024 - 2048 - xchg;
   if (half) p.kps = 1;
   const int stage_bytes = p.kps * kb_bytes;
   int max_stages = budget / stage_bytes;

@@ -91,3 +91,29 @@ def test_the_image_of_a_matrix_is_not_overwritten_by_the_next(which):
     for w, image in images:
         assert torch.equal(image, w.to(torch.bfloat16))
     assert len({image.untyped_storage().data_ptr() for _, image in images}) == len(images)
+
+
+@pytest.mark.parametrize("tokens,top,half", [(1, 2, False), (2, 2, False), (4, 2, False), (16, 2, True),
+                                             (1, 8, True), (32, 8, True)])
+def test_ring_of_an_expert_product_follows_the_groups_with_rows(launches, tokens, top, half):
+    """8 experts of 2 x 2752 x 2048: half the shared memory per CTA only where the CTAs that find rows
+    outnumber the SMs; otherwise stages of several k-blocks."""
+    T, E, F, K = tokens * top, 8, 2752, 2048
+    x, out = (OnGpu(torch.zeros(T, n, dtype=torch.bfloat16)) for n in (K, F))
+    w1, w3 = (OnGpu(torch.zeros(E * F, K, dtype=torch.bfloat16)) for _ in range(2))
+    off = torch.zeros(E + 1, dtype=torch.int32)
+    gemm.grouped_swiglu(x, w1, w3, out, off, E, tokens)
+    kps, stages, early, _ = _plan(launches[0])
+    assert not early and stages >= 2 and (kps == 1) == half
+
+
+@pytest.mark.parametrize("T", [1, 8, 64, 70, 128])
+@pytest.mark.parametrize("E,F,K", [(128, 128, 2048), (16, 1000, 4096), (300, 64, 512), (4, 11008, 1024)])
+def test_expert_products_keep_two_blocks_in_flight(launches, E, F, K, T):
+    """The exchange buffer of split sums counts against half a ring; many groups, few rows."""
+    x, out = (OnGpu(torch.zeros(T, n, dtype=torch.bfloat16)) for n in (K, F))
+    w1, w3 = (OnGpu(torch.zeros(E * F, K, dtype=torch.bfloat16)) for _ in range(2))
+    off = torch.zeros(E + 1, dtype=torch.int32)
+    gemm.grouped_swiglu(x, w1, w3, out, off, E, T)
+    kps, stages, _, _ = _plan(launches[0])
+    assert kps * stages >= 2
