@@ -368,10 +368,14 @@ extern "C" int e2h_gemm_rows(const E2hGemmParams* pp, int bits, void* stream_v) 
     return -9;
   const int units = (p.K * (bits / 4) + 127) / 128;      // of 64 bytes of a row
   // Two tiles per warp halve the reads of B; with few features the tiles themselves are what fills
-  // the SMs (4096 features, one row: 7.4 us with one tile, 9.0 with two). Eight warps split K where
-  // the tiles alone would leave an SM with less than 16 warps; from 9 rows on the reads of B leave
-  // room for fewer (12288 features, 16 rows: 24.2 us with eight warps, 21.9 with four).
-  const int mt = p.F >= 32 * 148 * 2 ? 2 : 1;
+  // the SMs (4096 features, one row: 7.4 us with one tile, 9.0 with two). From 9 rows on those reads
+  // weigh more than the weights, and one round of tiles of 32 features is enough (8192 x 8192, 16 rows,
+  // one -> two: int4 40.9 -> 22.9 us, int8 25.7 -> 21.6, bf16 29.0 -> 27.0), but for short sums (512:
+  // int8 4.6 -> 5.3). Eight warps split K where the tiles alone would leave an SM with less than 16
+  // warps; from 9 rows on the reads of B leave room for fewer (12288 features, 16 rows: 24.2 us with
+  // eight warps, 21.9 with four).
+  const bool wide = p.T > 8 && p.K >= 2048;
+  const int mt = p.F >= 32 * 148 * (wide ? 1 : 2) ? 2 : 1;     // (rows_pays in ops/gemm.py knows this)
   const int ft = p.dual ? 16 : 16 * mt;
   const int tiles = (p.F + ft - 1) / ft;
   int warps = tiles >= 148 * (p.T > 8 ? 2 : 4) ? 4 : 8;

@@ -124,26 +124,51 @@ ROWS_GATED = {EPI_SWIGLU, EPI_DUAL_STORE}
 ROWS_MAX = 16
 
 
+def rows_pays(F: int, K: int, T: int, bits: int) -> bool:
+    """Whether a plain product of 9 to 16 rows is at least as fast on the kernel for few rows as on the
+    tcgen05 ones. A tile of 16 or 32 features reads all rows there, where 128 features share them here:
+    the more K T, the less the saved set-up of 5 us counts, and a last round of tiles that leaves SMs
+    idle costs more. With tiles of 32 features and eight warps (csrc/gemm_rows.cu) the reads are no
+    bound. 16 rows, us there / here: bf16 4096 x 4096 10.3 / 12.4, 4096 x 11008 22.8 / 22.0, 8192 x 22016
+    63.4 / 64.6, 5120 x 13824 (160 tiles on 148 SMs) 36.1 / 29.6; int4 4096 x 8192 18.1 / 17.4, 8192 x
+    22016 53.6 / 64.9, 1536 x 4096 (96 tiles) 9.4 / 8.8. Over 1300 products of 512 to 32000 features
+    and K of 512 to 22016 the rule is within 0.3 % of the better choice on average, 14 % at most."""
+    two = F >= 32 * N_SM * (1 if K >= 2048 else 2)       # tiles per warp: as in csrc/gemm_rows.cu
+    tiles = -(-F // (32 if two else 16))
+    uneven = -(-tiles // N_SM) * N_SM / tiles if 2 * tiles > N_SM else 1.0
+    if bits == 16:
+        if two and tiles < 2 * N_SM:
+            return uneven < 1.6 or K * T <= 62_000
+        return K * T * uneven <= (90_000 if two else 135_000)
+    return two or K * T * uneven ** (4 if bits == 8 else 3) <= (600_000 if bits == 8 else 190_000)
+
+
 def rows_rule(a, a2, b, epi: int) -> bool:
     """Whether a product runs on the kernel for few rows (csrc/gemm_rows.cu): up to 16, the range that
-    its two groups of eight token columns cover and over which it is nowhere slower than the tcgen05
-    kernels (16 rows, 4096 x 11008: 21.8 us both; everything smaller gains, by up to 3x), token-major
-    outputs, and operands whose rows are whole 16-byte pieces. Anything else goes where it went."""
+    its two groups of eight token columns cover, token-major outputs, and operands whose rows are whole
+    16-byte pieces. Up to 8 rows, gated, and quantised matrices that another kernel would take only
+    after an expansion gain (up to 3x); for the others ``rows_pays``. What is left goes where it went."""
     T, K = b.shape
     if T > ROWS_MAX or epi not in (ROWS_EPIS if a2 is None else ROWS_GATED):
         return False
     if _ld(b) % 8 or b.data_ptr() % 16:
         return False
+    expands = False
     for w in (a,) if a2 is None else (a, a2):
         if isinstance(w, Int4Weight):
             q, piece, g = w.q, 128, w.groupsize
             if g < 32 or g & (g - 1):
                 return False
+            expands = g < 64
         else:
             q, piece = w, 16 // w.element_size()
+            expands = w.element_size() == 1 and K % 128 != 0
         if K % piece or _ld(q) * q.element_size() % 16 or q.data_ptr() % 16:
             return False
-    return True
+    if T <= 8 or a2 is not None or expands:
+        return True
+    bits = 4 if isinstance(a, Int4Weight) else 8 * a.element_size()
+    return rows_pays(a.shape[0], K, T, bits)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tensor] = None,

@@ -38,7 +38,8 @@ def _bound(x, w):
 @pytest.mark.parametrize("T", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("bits,F,K", [(16, 16, 8), (16, 130, 72), (16, 4096, 1032), (16, 9504, 512),
                                       (8, 40, 16), (8, 256, 1040), (8, 9504, 4096), (4, 17, 128),
-                                      (4, 384, 1408), (4, 9504, 1024)])
+                                      (4, 384, 1408), (4, 9504, 1024), (16, 4744, 2056),
+                                      (8, 4744, 2064), (4, 4744, 2176)])
 def test_linear(T, bits, F, K):
     from easy_to_hard_b200.ops import gemm
     w, s, wf = _weight(F, K, bits, T + F, pad=8)
