@@ -14,11 +14,16 @@
 // so only the handful of entries at or above it are collected (typically 50-70 of 32016) and
 // the pivot is picked among them by rank counting; the sampling pass then also runs over those
 // candidates only. The group maxima are taken while the row is copied, four threads rank a maximum
-// and the candidate pass reads 16 bytes at a time: 32 rows of 32000: 12.8 -> 9.0 us. Otherwise, or if more than 2048 entries reach the bound (many equal logits):
-// a 4-pass, 8-bit radix select over the order-preserving integer image of the fp32 logits. The row (128 KB at a 32k vocabulary) is
-// copied into shared memory once with 16-byte loads and all five passes read it from there: the
-// passes are chains of dependent loads (a warp-wide match between them), which from L2 cost
-// ~13 us per pass and ~100 us per step; rows that do not fit stay in global memory.
+// and the candidate pass reads 16 bytes at a time: 32 rows of 32000: 12.8 -> 9.0 us. Neighbouring
+// 16-byte pieces (elements, where a group would go without) go to different groups, so that no group is
+// empty or much smaller than another: with neighbouring pieces in one group fewer groups than top_k
+// had entries in a small vocabulary, and every entry became a candidate (2000 logits, top 200: 151
+// us, 11 now). Otherwise, or if more than 1024 entries reach the bound (many equal logits, top_k
+// near 256; ranking 1400 candidates takes 77 to 150 us, the passes 44 over 32000 logits): a 4-pass, 8-bit radix
+// select over the order-preserving integer image of the fp32 logits. The row (128 KB at a 32k
+// vocabulary) is copied into shared memory once and all five passes read it from there: the passes
+// are chains of dependent loads (a warp-wide match between them), which from L2 cost ~13 us per pass
+// and ~100 us per step; rows that do not fit stay in global memory.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -50,7 +55,7 @@ __device__ __forceinline__ uint4 philox(uint4 ctr, uint2 key) {
 constexpr int kSampThreads = 1024;
 constexpr int kSampMaxSmemRow = 188 * 1024;     // bytes of one logits row kept in shared memory
 constexpr int kSampGroups = 256;                // group maxima of the fast path
-constexpr int kSampCandMax = 2048;              // candidates the fast path can hold
+constexpr int kSampCandMax = 1024;              // candidates of the fast path: one per thread
 
 // logits   : fp32 [B, ld]
 // pos_ptr  : device scalar, position of the token that produced these logits; the sampled
@@ -84,15 +89,18 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
   const float* row = logits + (long long)b * ld;
   pdl_wait_prior();
   pdl_launch_dependents();
-  // the row goes to shared memory, and every thread keeps the largest key that it moved
+  // the row goes to shared memory, and every thread keeps the largest key that it moved. Four lanes of a
+  // warp, 8 apart, make a group; group g takes the elements (16-byte pieces) g, g + 256, g + 512, ...
   uint32_t lm = 0;
+  const int group = (threadIdx.x >> 5) * 8 + (threadIdx.x & 7), part = (threadIdx.x >> 3) & 3;
+  const int first_elem = group + kSampGroups * part;
   if (threadIdx.x == 0) n_cand = 0;
   if (row_in_smem) {
-    if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    if ((reinterpret_cast<uintptr_t>(row) & 15) == 0 && vocab >= 4 * kSampGroups) {
       const float4* src4 = reinterpret_cast<const float4*>(row);
       float4* dst4 = reinterpret_cast<float4*>(srow);
 #pragma unroll 4
-      for (int i = threadIdx.x; i < vocab / 4; i += kSampThreads) {
+      for (int i = first_elem; i < vocab / 4; i += kSampThreads) {
         const float4 v = src4[i];
         dst4[i] = v;
         lm = max(lm, max(max(float_key(v.x), float_key(v.y)), max(float_key(v.z), float_key(v.w))));
@@ -102,7 +110,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
         lm = max(lm, float_key(row[i]));
       }
     } else {
-      for (int i = threadIdx.x; i < vocab; i += kSampThreads) {
+      for (int i = first_elem; i < vocab; i += kSampThreads) {
         srow[i] = row[i];
         lm = max(lm, float_key(row[i]));
       }
@@ -118,10 +126,9 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
   uint32_t pivot_key = 0;  // keep everything
   bool have_cands = false; // the entries >= pivot_key are (among) the first n_cand candidates
   if (!greedy && top_k > 0 && top_k < vocab && row_in_smem && top_k <= kSampGroups) {
-    // ---- fast path: four neighbouring threads make a group
-    lm = max(lm, __shfl_xor_sync(0xffffffffu, lm, 1));
-    lm = max(lm, __shfl_xor_sync(0xffffffffu, lm, 2));
-    const int group = threadIdx.x >> 2, part = threadIdx.x & 3;
+    // ---- fast path
+    lm = max(lm, __shfl_xor_sync(0xffffffffu, lm, 8));
+    lm = max(lm, __shfl_xor_sync(0xffffffffu, lm, 16));
     if (part == 0) gmax[group] = lm;
     __syncthreads();
     // rank of this group's maximum among the 256 (ties broken by group index), a quarter of them per
@@ -135,8 +142,8 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
 #pragma unroll
       for (int e = 0; e < 4; ++e) gt += (w[e] > lm || (w[e] == lm && first + e < group)) ? 1 : 0;
     }
-    gt += __shfl_xor_sync(0xffffffffu, gt, 1);
-    gt += __shfl_xor_sync(0xffffffffu, gt, 2);
+    gt += __shfl_xor_sync(0xffffffffu, gt, 8);
+    gt += __shfl_xor_sync(0xffffffffu, gt, 16);
     if (part == 0 && gt == top_k - 1) sh_bound = lm;
     __syncthreads();
     const uint32_t bound = sh_bound;

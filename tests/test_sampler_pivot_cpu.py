@@ -7,15 +7,20 @@ import pytest
 THREADS, GROUPS = 1024, 256
 
 
-def _pivot_by_candidates(row: np.ndarray, k: int):
+def _pivot_by_candidates(row: np.ndarray, k: int, aligned: bool = True):
     v = len(row)
-    # per-thread maxima over a strided walk, then per-group maxima (threads t, t + 256, ...)
-    tmax = np.full(THREADS, -np.inf)
-    for t in range(THREADS):
-        part = row[t::THREADS]
-        if len(part):
-            tmax[t] = part.max()
-    gmax = tmax.reshape(THREADS // GROUPS, GROUPS).max(axis=0)
+    # group g takes the 16-byte pieces g, g + 256, ..., or the elements where a group would get no piece;
+    # the ragged end goes to the first threads
+    gmax = np.full(GROUPS, -np.inf)
+    piece = 4 if aligned and v >= 4 * GROUPS else 1
+    body = v // piece * piece
+    for g in range(GROUPS):
+        mine = row[:body].reshape(-1, piece)[g::GROUPS]
+        if mine.size:
+            gmax[g] = mine.max()
+    for t, x in enumerate(row[body:]):
+        g = (t >> 5) * 8 + (t & 7)
+        gmax[g] = max(gmax[g], x)
     # rank by (value desc, group index asc): the group of rank k - 1 gives the bound
     order = sorted(range(GROUPS), key=lambda j: (-gmax[j], j))
     bound = gmax[order[k - 1]]
@@ -38,5 +43,18 @@ def test_candidate_pivot_is_the_kth_largest(seed, k):
     pivot, n_cand, _ = _pivot_by_candidates(row, k)
     assert pivot == np.sort(row)[-k]
     assert n_cand >= k
-    if seed % 3:
-        assert n_cand <= 2048               # the list the kernel keeps is long enough
+    if seed % 3 and k < 256:
+        assert n_cand <= 1024               # the list the kernel keeps is long enough
+
+
+@pytest.mark.parametrize("v", [500, 1000, 1024, 2000, 4000, 4096, 5003])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_small_vocabularies_leave_few_candidates(v, aligned):
+    """No group is empty where there are 256 elements: with as many groups as top_k or more the bound
+    still drops most of the row."""
+    for seed in range(6):
+        row = np.random.default_rng(seed).standard_normal(v).astype(np.float32)
+        for k, share in ((50, 0.25), (200, 0.8)):
+            pivot, n_cand, _ = _pivot_by_candidates(row, k, aligned)
+            assert pivot == np.sort(row)[-k]
+            assert n_cand <= share * v
