@@ -162,6 +162,50 @@ __device__ __forceinline__ void attn_chunk_mma(const uint8_t* ks, const uint8_t*
   }
 }
 
+// The output of a run once more, for runs whose values were not all finite: an infinite value times a
+// part of a probability that is 0 is NaN, although the probability as a whole is not 0. Whole fp32
+// probabilities here, on the CUDA cores and from global memory; m is the run's maximum of this warp's
+// keys. Never inlined and writing to shared memory, so that the fast path keeps its registers
+// (a check of every fragment there cost up to 13 %).
+template <int G>
+__device__ __noinline__ void attn_run_plain(const __nv_bfloat16* q, const __nv_bfloat16* k,
+                                            const __nv_bfloat16* v, int n_keys, int warp, int lane,
+                                            float scale, float m, float* acc) {
+  const int g = lane >> 2, t = lane & 3;
+  float o[16][2];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = 0.f;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  for (int first = 8 * warp; first < n_keys; first += 32) {
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const uint4 a = g < G ? *reinterpret_cast<const uint4*>(q + g * 128 + 32 * d + 8 * t) : none;
+      const uint4 b = first + g < n_keys
+                          ? *reinterpret_cast<const uint4*>(k + (first + g) * 128 + 32 * d + 8 * t)
+                          : none;
+      mma_16816(c, a.x, 0u, a.y, 0u, b.x, b.y);
+      mma_16816(c, a.z, 0u, a.w, 0u, b.z, b.w);
+    }
+    for (int u = 0; u < 8 && first + u < n_keys; ++u) {
+      const float s = __shfl_sync(0xffffffffu, (u & 1) ? c[1] : c[0], (lane & ~3) | (u >> 1));
+      const float w = __expf(s * scale - m);
+      const __nv_bfloat16* row = v + (first + u) * 128 + 2 * t;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + 8 * i));
+        o[i][0] += w * x.x;
+        o[i][1] += w * x.y;
+      }
+    }
+  }
+  if (g < G) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      *reinterpret_cast<float2*>(acc + g * 128 + 8 * i + 2 * t) = make_float2(o[i][0], o[i][1]);
+  }
+}
+
 // D = 16 * 8 * R : each lane of the half-warp holds R groups of 8 consecutive elements.
 template <int D, int G>
 __global__ void __launch_bounds__(kAttnThreads, AttnForm<D, G>::mma ? 3 : 0)
@@ -377,6 +421,17 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
           sm_m[warp][g] = m;
           sm_l[warp][g] = l;
         }
+      }
+      float all = 0.f;                     // 0, or NaN if a sum is not finite
+#pragma unroll
+      for (int i = 0; i < 16; ++i) all = fmaf(o[i][0], 0.f, fmaf(o[i][1], 0.f, all));
+      if (__any_sync(0xffffffffu, all != 0.f) && !dead) {
+        const int key0 = w.start + w.ch * kChunk;
+        const long long row0 = ((long long)(w.b * n_kv + w.hk) * smax + key0) * D;
+        attn_run_plain<G>(q + ((long long)w.b * n_head + w.hk * G) * D, kcache + row0, vcache + row0,
+                          min(n_here * kChunk, pos + 1 - key0), warp, lane, scale, m,
+                          &sm_acc[warp][0][0]);
+      } else if (g < G) {
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           *reinterpret_cast<float2*>(&sm_acc[warp][g][8 * i + 2 * t]) = make_float2(o[i][0], o[i][1]);

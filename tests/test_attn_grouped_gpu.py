@@ -60,3 +60,31 @@ def test_a_captured_step_survives_a_larger_batch():
         assert torch.equal(out, want)
     assert all(bool((t == -1).all()) for t in taken)
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("G", [4, 8])
+@pytest.mark.parametrize("n_split", [1, 8])
+def test_infinite_values_stay_infinite(G, n_split):
+    """The probabilities are split into parts, of which some are 0: an infinite value must not meet
+    these. Dims without one keep their bound."""
+    from easy_to_hard_b200.ops import _lib, functional as Fn
+    B, n_kv, D, smax, pos = 3, 2, 128, 128, 100
+    g = torch.Generator(device="cuda").manual_seed(G)
+    q = torch.randn(B, n_kv * G * D, device="cuda", generator=g).bfloat16()
+    q[1] = 0                                        # equal probabilities: exact in the first part
+    kc, vc = (torch.randn(B, n_kv, smax, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    vc[:, :, 3, 5], vc[:, 1, 40, 6], vc[:, 0, 100, 127] = float("inf"), float("-inf"), float("inf")
+    vc[2, 1, 60, 8], vc[2, 1, 61, 8], vc[0, 0, 9, 9] = float("inf"), float("-inf"), float("nan")
+    at = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    out = Fn.attn_decode(q, kc, vc, at, None, n_kv * G, n_split=n_split).view(B, n_kv * G, D)
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+    k, v = (t[:, :, :pos + 1].double().repeat_interleave(G, 1) for t in (kc, vc))
+    s = (k @ q.double().view(B, n_kv * G, D, 1))[..., 0] * D ** -0.5
+    want = (torch.softmax(s, -1)[..., None] * v).sum(2)
+    live = torch.isfinite(want)
+    assert int((~live).sum()) > 0 and torch.equal(torch.isfinite(out), live)
+    assert torch.equal(torch.isnan(out), torch.isnan(want))
+    assert torch.equal(out[torch.isinf(want)].double(), want[torch.isinf(want)])
+    err = (out.double() - want).abs()
+    assert bool((err[live] <= (2.0 ** -8 * want.abs() + 2.0 ** -17 * 8)[live]).all())
