@@ -15,12 +15,12 @@
 // the pivot is picked among them by rank counting; the sampling pass then also runs over those
 // candidates only. The group maxima are taken while the row is copied, four threads rank a maximum
 // and the candidate pass reads 16 bytes at a time: 32 rows of 32000: 12.8 -> 9.0 us. Neighbouring
-// 16-byte pieces (elements, where a group would go without) go to different groups, so that no group is
-// empty or much smaller than another: with neighbouring pieces in one group fewer groups than top_k
-// had entries in a small vocabulary, and every entry became a candidate (2000 logits, top 200: 151
+// 16-byte pieces of a small vocabulary (elements, where a group would go without) go to different
+// groups, so that no group is empty or much smaller than another: with neighbours in one group,
+// fewer groups than top_k had entries, and every entry became a candidate (2000 logits, top 200: 151
 // us, 11 now). Otherwise, or if more than 1024 entries reach the bound (many equal logits, top_k
-// near 256; ranking 1400 candidates takes 77 to 150 us, the passes 44 over 32000 logits): a 4-pass, 8-bit radix
-// select over the order-preserving integer image of the fp32 logits. The row (128 KB at a 32k
+// near 256; ranking 1400 candidates takes 77 to 150 us, the passes 44 over 32000 logits): a 4-pass,
+// 8-bit radix select over the order-preserving integer image of the fp32 logits. The row (128 KB at a 32k
 // vocabulary) is copied into shared memory once and all five passes read it from there: the passes
 // are chains of dependent loads (a warp-wide match between them), which from L2 cost ~13 us per pass
 // and ~100 us per step; rows that do not fit stay in global memory.
@@ -90,13 +90,17 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
   pdl_wait_prior();
   pdl_launch_dependents();
   // the row goes to shared memory, and every thread keeps the largest key that it moved. Four lanes of a
-  // warp, 8 apart, make a group; group g takes the elements (16-byte pieces) g, g + 256, g + 512, ...
+  // warp, 8 apart, make a group. In a small vocabulary group g takes the elements (16-byte pieces) g,
+  // g + 256, g + 512, ...; a large one is copied in the order of the threads, a warp 512 bytes at a
+  // time (32 rows of 32000: 9.4 -> 9.0 us)
   uint32_t lm = 0;
   const int group = (threadIdx.x >> 5) * 8 + (threadIdx.x & 7), part = (threadIdx.x >> 3) & 3;
-  const int first_elem = group + kSampGroups * part;
+  const bool spread = temperature > 0.f && top_k > 0 && vocab < 16 * kSampThreads;
+  const int first_elem = spread ? group + kSampGroups * part : (int)threadIdx.x;
   if (threadIdx.x == 0) n_cand = 0;
   if (row_in_smem) {
-    if ((reinterpret_cast<uintptr_t>(row) & 15) == 0 && vocab >= 4 * kSampGroups) {
+    if ((reinterpret_cast<uintptr_t>(row) & 15) == 0 &&
+        (!spread || vocab >= 4 * kSampGroups)) {
       const float4* src4 = reinterpret_cast<const float4*>(row);
       float4* dst4 = reinterpret_cast<float4*>(srow);
 #pragma unroll 4

@@ -10,17 +10,18 @@ THREADS, GROUPS = 1024, 256
 def _pivot_by_candidates(row: np.ndarray, k: int, aligned: bool = True):
     v = len(row)
     # group g takes the 16-byte pieces g, g + 256, ..., or the elements where a group would get no piece;
-    # the ragged end goes to the first threads
+    # a large vocabulary goes round the threads, of which four lanes 8 apart make a group, and so does
+    # the ragged end
     gmax = np.full(GROUPS, -np.inf)
-    piece = 4 if aligned and v >= 4 * GROUPS else 1
+    spread = v < 16 * THREADS
+    piece = 4 if aligned and (not spread or v >= 4 * GROUPS) else 1
     body = v // piece * piece
-    for g in range(GROUPS):
-        mine = row[:body].reshape(-1, piece)[g::GROUPS]
-        if mine.size:
-            gmax[g] = mine.max()
-    for t, x in enumerate(row[body:]):
-        g = (t >> 5) * 8 + (t & 7)
-        gmax[g] = max(gmax[g], x)
+    top = row[:body].reshape(-1, piece).max(axis=1)
+    t = np.arange(len(top)) % THREADS
+    at = np.arange(len(top)) % GROUPS if spread else (t >> 5) * 8 + (t & 7)
+    np.maximum.at(gmax, at, top)
+    t = np.arange(v - body)
+    np.maximum.at(gmax, (t >> 5) * 8 + (t & 7), row[body:])
     # rank by (value desc, group index asc): the group of rank k - 1 gives the bound
     order = sorted(range(GROUPS), key=lambda j: (-gmax[j], j))
     bound = gmax[order[k - 1]]
