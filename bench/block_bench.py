@@ -37,7 +37,7 @@ def main():
     pos = torch.arange(S, device=dev, dtype=torch.int32).repeat(B)
     x = torch.randn(T, dim, device=dev).bfloat16()
     dy = torch.randn(T, dim, device=dev).bfloat16()
-    shape = fb.BlockShape(B, S, H, H, D, 1e-5)
+    shape = fb.BlockShape(B, S, H, H, D, 1e-5, in_order=True)
     grads = {k: torch.empty_like(v) for k, v in w.items() if k.startswith('w')}
     def t(fn, n=5):
         for _ in range(2): fn()

@@ -36,6 +36,7 @@ class BlockShape:
     eps: float
     tp: int = 1
     sequence_parallel: bool = False
+    in_order: bool = False    # the positions of every sequence are consecutive from pos[0] on
 
 
 def _tp_all_reduce(t: torch.Tensor, shape: BlockShape) -> torch.Tensor:
@@ -140,9 +141,8 @@ def _row_parallel_fused(x_in: torch.Tensor, w: torch.Tensor, residual: torch.Ten
 def block_forward(x: torch.Tensor, w: Dict[str, torch.Tensor], freqs: torch.Tensor,
                   pos: torch.Tensor, shape: BlockShape, keep: bool = False):
     """x [T, dim] (T = B*S, or B*S/tp rows under sequence parallelism). ``w`` holds bf16
-    ``wqkv, wo, w1, w3, w2`` and the two norm weights; ``pos`` the positions of the B*S tokens, those
-    of a sequence consecutive and every sequence from the same one on. Returns ``out`` and, with
-    ``keep``, the intermediates the backward needs."""
+    ``wqkv, wo, w1, w3, w2`` and the two norm weights; ``pos`` int32 the positions of the B*S tokens.
+    Returns ``out`` and, with ``keep``, the intermediates the backward needs."""
     H, Hkv, D = shape.n_head, shape.n_kv, shape.head_dim
     sp = shape.sequence_parallel and shape.tp > 1
     fused_sp = sp and p2p_reduce_enabled()
@@ -157,10 +157,13 @@ def block_forward(x: torch.Tensor, w: Dict[str, torch.Tensor], freqs: torch.Tens
         xn1 = Fn.rmsnorm(x, w["attention_norm"], shape.eps)
         xn1f = _sp_gather(xn1, shape) if sp else xn1
     T = xn1f.shape[0]
-    # q and k heads rotated in the epilogue; the rows are whole sequences from position pos[0] on
-    qkv = gemm.linear_qkv_rope(xn1f, w["wqkv"], torch.empty(
-        T, (H + 2 * Hkv) * D, dtype=xn1f.dtype, device=xn1f.device), freqs=freqs, pos_base=pos,
-        sq=shape.S, n_head=H, n_kv=Hkv, head_dim=D)
+    if shape.in_order:             # q and k heads rotated in the epilogue
+        qkv = gemm.linear_qkv_rope(xn1f, w["wqkv"], torch.empty(
+            T, (H + 2 * Hkv) * D, dtype=xn1f.dtype, device=xn1f.device), freqs=freqs, pos_base=pos,
+            sq=shape.S, n_head=H, n_kv=Hkv, head_dim=D)
+    else:
+        qkv = gemm.linear(xn1f, w["wqkv"])
+        Fn.rope(qkv, freqs, pos, H + Hkv, D, out=qkv)      # in place
     q = qkv[:, : H * D].view(shape.B, shape.S, H, D)
     k = qkv[:, H * D: (H + Hkv) * D].view(shape.B, shape.S, Hkv, D)
     v = qkv[:, (H + Hkv) * D:].view(shape.B, shape.S, Hkv, D)
@@ -333,7 +336,7 @@ def transformer_hidden(model, idx: torch.Tensor, final_norm: bool = True) -> tor
         model.setup_caches(B, S, kv_cache=False)
     att = model.layers[0].attention
     shape = BlockShape(B, S, att.n_head, att.n_local_heads, att.head_dim, model.config.norm_eps,
-                       tp=getattr(att, "tp_size", 1), sequence_parallel=False)
+                       tp=getattr(att, "tp_size", 1), sequence_parallel=False, in_order=True)
     pos = torch.arange(S, device=idx.device, dtype=torch.int32).repeat(B)
     x = model.embed(idx).to(torch.bfloat16).reshape(B * S, -1)
     for blk in model.layers:

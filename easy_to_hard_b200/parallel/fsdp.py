@@ -420,7 +420,8 @@ class ShardedDataParallel(nn.Module):
         a = blk.attention
         return BlockShape(B, S, a.n_head, a.n_local_heads, a.head_dim, self.backbone.config.norm_eps,
                           tp=getattr(a, "tp_size", 1),
-                          sequence_parallel=getattr(a, "sequence_parallel", False))
+                          sequence_parallel=getattr(a, "sequence_parallel", False),
+                          in_order=True)
 
     def _run_block(self, idx: int, x: torch.Tensor, B: int, S: int, keep: bool = False):
         """One block forward. With ``keep`` (a training forward) the block's intermediates are
