@@ -157,7 +157,7 @@ def rows_rule(a, a2, b, epi: int) -> bool:
     for w in (a,) if a2 is None else (a, a2):
         if isinstance(w, Int4Weight):
             q, piece, g = w.q, 128, w.groupsize
-            if g < 32 or g & (g - 1):
+            if g < 32 or g & (g - 1) or not w.plain():
                 return False
             expands = g < 64
         else:
@@ -206,8 +206,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         assert not a_mn_major and not b_mn_major and tiled_shape is None and scale is None
         assert a2 is None or isinstance(a2, Int4Weight)
         K4 = a.shape[1]
-        if not rows and (b.shape[0] > 128 or K4 % 128 or a.groupsize < 64 or a.groupsize & (a.groupsize - 1)
-                         or (K4 // 2) % 16):
+        if not rows and (b.shape[0] > 128 or K4 % 128 or a.groupsize < 64
+                         or a.groupsize & (a.groupsize - 1) or (K4 // 2) % 16
+                         or not all(w.plain() for w in (a, a2) if w is not None)):
             a = _expand_int4(a, 0)            # many tokens: one dequantisation pass, then bf16
             a2 = _expand_int4(a2, 1) if a2 is not None else None
             w4, fresh = False, True
@@ -415,6 +416,13 @@ class Int4Weight:
         q = word.view(torch.uint8).view(F, K // 2).contiguous()
         return cls(q, sz.to(torch.bfloat16).contiguous(), groupsize, (F, K))
 
+    def plain(self) -> bool:
+        """Whether the (scale, zero) pairs lie as the kernels read them: dense bf16 [>= K / g, F, 2] on
+        4-byte boundaries. Any other layout goes through ``dequant``."""
+        sz, (F, K) = self.sz, self.shape
+        return (sz.dtype == torch.bfloat16 and sz.is_contiguous() and sz.data_ptr() % 4 == 0
+                and tuple(sz.shape[1:]) == (F, 2) and sz.shape[0] * self.groupsize >= K)
+
     def codes(self) -> torch.Tensor:
         """Integer codes [F, K] (inverse of ``from_int``)."""
         F, K = self.shape
@@ -460,7 +468,8 @@ def _expand_int4(w: "Int4Weight", which: int) -> torch.Tensor:
     """bf16 image of an int4 weight, as ``_expand_int8``."""
     out = torch.empty(w.shape, dtype=torch.bfloat16, device=w.device)
     F, K = w.shape
-    if w.groupsize % 8 == 0 and w.q.stride(1) == 1 and w.q.stride(0) % 4 == 0:
+    if (w.groupsize % 8 == 0 and w.plain() and w.q.stride(1) == 1 and w.q.stride(0) % 4 == 0
+            and w.q.data_ptr() % 4 == 0):
         _lib.check(_lib.lib().e2h_expand_weight(w.q.data_ptr(), w.q.stride(0), 4, w.sz.data_ptr(),
                                                 w.groupsize, out.data_ptr(), F, K, _lib.stream()),
                    "e2h_expand_weight")

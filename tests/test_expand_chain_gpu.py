@@ -110,3 +110,19 @@ def test_two_streams_expand_at_once():
         for i in range(20):
             _close(out[i], ref, x, wf)
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("T", [4, 64, 200])
+def test_strided_pairs(T):
+    from easy_to_hard_b200.ops import _lib, gemm
+    F, K, group = 96, 512, 64
+    dense, _, wf = _weight(F, K, 4, 5)
+    sz = torch.rand(K // group, F, 4, device="cuda").bfloat16()[..., ::2]
+    w = gemm.Int4Weight(dense.q, sz, group, (F, K))
+    wf = w.dequant().float()
+    assert torch.equal(gemm._expand_int4(w, 0), w.dequant())
+    x = torch.randn(T, K, device="cuda").bfloat16()
+    got = gemm.linear(x, w)
+    torch.cuda.synchronize()
+    _close(got, x.double() @ wf.double().t(), x, wf)
+    assert _lib.read_status() == 0

@@ -117,3 +117,33 @@ def test_expert_products_keep_two_blocks_in_flight(launches, E, F, K, T):
     gemm.grouped_swiglu(x, w1, w3, out, off, E, T)
     kps, stages, _, _ = _plan(launches[0])
     assert kps * stages >= 2
+
+
+@pytest.mark.parametrize("T", [4, 16, 64, 200])
+def test_int4_pairs_of_another_layout_go_through_the_general_expansion(launches, monkeypatch, T):
+    """The kernels read (scale, zero) pairs as dense bf16: strided, fp32 or odd ones are dequantised."""
+    F, K, g = 24, 256, 64
+    codes = torch.randint(0, 16, (F, K), dtype=torch.int32)
+    sz = torch.rand(K // g, F, 2).bfloat16()
+    good = gemm.Int4Weight.from_int(codes, sz, g)
+    apart = torch.zeros(K // g, F, 4).bfloat16()
+    apart[..., ::2] = sz
+    odd = torch.zeros(sz.numel() + 1).bfloat16()[1:].view(sz.shape)
+    odd.copy_(sz)
+    expanded = []
+
+    def expand(w, which):
+        expanded.append(w.dequant().bfloat16())
+        return OnGpu(expanded[-1])
+    monkeypatch.setattr(gemm, "_expand_int4", expand)
+    x, out = (OnGpu(torch.zeros(T, n, dtype=torch.bfloat16)) for n in (K, F))
+    assert good.plain()
+    for pairs in (apart[..., ::2], sz.permute(1, 0, 2).contiguous().permute(1, 0, 2), odd, sz.float()):
+        w = gemm.Int4Weight(good.q, pairs, g, (F, K))
+        w.is_cuda = True
+        assert not w.plain()
+        del expanded[:], launches[:]
+        if T > 16:          # (below, a bf16 image takes the kernel for few rows, which is not recorded)
+            gemm.linear(x, w, out=out)
+            assert len(launches) == 1 and len(expanded) == 1
+        assert not gemm.rows_rule(w, None, x, gemm.EPI_STORE_BF16)
