@@ -678,31 +678,18 @@ static int launch_decode(const void* q, const void* k, const void* v, void* out,
     const char* e = getenv("E2H_ATTN_L2HINT");
     return e && e[0] == '0';
   }();
-  // more than 48 KB of dynamic shared memory has to be asked for once per device
-  static std::mutex mu;
-  static bool asked[64];
-  static int n_sm[64];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  static SmemAsk ask;
+  cudaError_t e = ask(attn_decode_kernel<D, G>, attn_smem_bytes(D, kAttnMaxStages));
   if (e != cudaSuccess) return (int)e;
-  if (dev < 0 || dev >= 64) return -5;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!asked[dev]) {
-      e = cudaFuncSetAttribute(attn_decode_kernel<D, G>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               attn_smem_bytes(D, kAttnMaxStages));
-      if (e != cudaSuccess) return (int)e;
-      e = cudaDeviceGetAttribute(&n_sm[dev], cudaDevAttrMultiProcessorCount, dev);
-      if (e != cudaSuccess) return (int)e;
-      asked[dev] = true;
-    }
-  }
+  int dev = 0, n_sm = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return (int)e;
   if (max_parts > kAttnMaxParts) max_parts = kAttnMaxParts;
   const long long q_stride = (long long)n_head * D;
   for (int b0 = 0; b0 < B; b0 += kAttnMaxB) {     // batches beyond kAttnMaxB go in slices
     const int nb = B - b0 < kAttnMaxB ? B - b0 : kAttnMaxB;
-    const int resident = n_sm[dev] * attn_ctas_per_sm(D, G, stages);
+    const int resident = n_sm * attn_ctas_per_sm(D, G, stages);
     int fixed_parts = 0;
     if (max_parts <= 1) {
       fixed_parts = 1;

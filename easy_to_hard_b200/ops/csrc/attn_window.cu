@@ -24,7 +24,6 @@
 #include <float.h>
 #include <stdint.h>
 #include <string.h>
-#include <mutex>
 
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -783,15 +782,9 @@ extern "C" int e2h_attn_prep(const e2h::AttnWindowParams* p, int is_bf16, void* 
                                  (cudaStream_t)stream, *p);
   const size_t smem = (size_t)(p->H + p->G) * p->dim * 4;
   if (smem > 200 * 1024) return -2;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [] {
-    err = cudaFuncSetAttribute(attn_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               200 * 1024);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(attn_prep_kernel<__nv_bfloat16>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
+  static SmemAsk ask_f32, ask_bf16;
+  const cudaError_t err = is_bf16 ? ask_bf16(attn_prep_kernel<__nv_bfloat16>, 200 * 1024)
+                                  : ask_f32(attn_prep_kernel<float>, 200 * 1024);
   if (err != cudaSuccess) return (int)err;
   return is_bf16 ? (int)launch(attn_prep_kernel<__nv_bfloat16>, dim3(p->n), dim3(256), smem,
                                (cudaStream_t)stream, *p)

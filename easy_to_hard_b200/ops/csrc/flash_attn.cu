@@ -23,9 +23,9 @@
 #include <cuda_bf16.h>
 #include <float.h>
 #include <string.h>
-#include <mutex>
 
 #include "flash_common.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace e2h {
@@ -862,22 +862,14 @@ extern "C" int e2h_flash_fwd(const void* q, long long q_sb, long long q_ss, long
   const size_t smem = 1024 + 2048 + 5 * (size_t)tile + 2 * (2 * 128 * 128);
   cudaError_t e;
   if (D == 128) {
-    static bool done = false;
-    if (!done) {
-      e = cudaFuncSetAttribute(flash_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-      if (e != cudaSuccess) return (int)e;
-      done = true;
-    }
+    static SmemAsk ask;
+    e = ask(flash_fwd_kernel<128>, smem);
+    if (e != cudaSuccess) return (int)e;
     flash_fwd_kernel<128><<<grid, kFwdThreads, smem, (cudaStream_t)stream>>>(tq, tk, tv, p);
   } else {
-    static bool done = false;
-    if (!done) {
-      e = cudaFuncSetAttribute(flash_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-      if (e != cudaSuccess) return (int)e;
-      done = true;
-    }
+    static SmemAsk ask;
+    e = ask(flash_fwd_kernel<64>, smem);
+    if (e != cudaSuccess) return (int)e;
     flash_fwd_kernel<64><<<grid, kFwdThreads, smem, (cudaStream_t)stream>>>(tq, tk, tv, p);
   }
   return (int)cudaGetLastError();
@@ -924,16 +916,10 @@ extern "C" int e2h_flash_bwd(const void* q, long long q_sb, long long q_ss, long
   cudaError_t e;
 #define E2H_BWD(D_)                                                                              \
   {                                                                                              \
-    static bool done = false;                                                                    \
-    if (!done) {                                                                                 \
-      e = cudaFuncSetAttribute(flash_bwd_dkdv_kernel<D_>,                                        \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv);       \
-      if (e != cudaSuccess) return (int)e;                                                       \
-      e = cudaFuncSetAttribute(flash_bwd_dq_kernel<D_>,                                          \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q);        \
-      if (e != cudaSuccess) return (int)e;                                                       \
-      done = true;                                                                               \
-    }                                                                                            \
+    static SmemAsk ask_kv, ask_q;                                                                \
+    e = ask_kv(flash_bwd_dkdv_kernel<D_>, smem_kv);                                              \
+    if (e == cudaSuccess) e = ask_q(flash_bwd_dq_kernel<D_>, smem_q);                            \
+    if (e != cudaSuccess) return (int)e;                                                         \
     flash_bwd_dkdv_kernel<D_><<<gkv, kFwdThreads, smem_kv, stream>>>(tq, tk, tv, tdo, p);                \
     flash_bwd_dq_kernel<D_><<<gq, kFwdThreads, smem_q, stream>>>(tq, tk, tv, tdo, p);                    \
   }

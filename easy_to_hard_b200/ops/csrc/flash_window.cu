@@ -31,7 +31,6 @@
 #include <float.h>
 #include <limits.h>
 #include <string.h>
-#include <mutex>
 
 #include "flash_common.cuh"
 #include "launch.cuh"
@@ -392,12 +391,8 @@ static int flash_window_launch(const FlashWindowMaps& m, const FlashWindowParams
                                cudaStream_t stream) {
   const size_t smem = 1024 + 2048 + (size_t)(3 * (KN + KR) + 2 * VH) * 128 * 128;
   static_assert(1024 + 2048 + (3 * (KN + KR) + 2 * VH) * 128 * 128 <= 227 * 1024, "shared memory");
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(flash_window_kernel<KN, KR, VH>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(flash_window_kernel<KN, KR, VH>, smem);
   if (err != cudaSuccess) return (int)err;
   return (int)launch(flash_window_kernel<KN, KR, VH>, grid, dim3(kWThreads), smem, stream, m.q,
                      m.q2, m.k, m.k2, m.v, p);

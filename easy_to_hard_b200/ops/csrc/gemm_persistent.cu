@@ -771,13 +771,9 @@ static int p_launch(E2hGemmParams& p, cudaStream_t stream) {
   p.stages = stages;
   const size_t smem = 2048 + (size_t)stages * STAGE + 4 * kChunkBytes;
   auto kern = umma_gemm_persistent_kernel<BN, DUAL, PAIR, SWI>;
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = smem;
-  }
+  static SmemAsk ask;
+  const cudaError_t granted = ask(kern, smem);
+  if (granted != cudaSuccess) return (int)granted;
   int n_sm = 148;
   {
     static int cached = 0;

@@ -32,7 +32,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
-#include <atomic>
 
 #include "gemm_epilogue.cuh"
 #include "gemm_umma.cuh"
@@ -302,18 +301,9 @@ static int rows_launch(const E2hGemmParams& p, int warps, cudaStream_t stream) {
   const int ft = DUAL ? 16 : 16 * MT;
   auto kern = gemm_rows_kernel<QB, MT, NT, DUAL>;
   constexpr int warp_bytes = RowsRing<QB, MT, NT>::bytes;
-  // more than 48 KB of dynamic shared memory has to be asked for once per device
-  static std::atomic<bool> asked[64];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  static SmemAsk ask;
+  const cudaError_t e = ask(kern, kRowsMaxWarps * warp_bytes);
   if (e != cudaSuccess) return (int)e;
-  if (dev < 0 || dev >= 64) return -10;
-  if (!asked[dev].load(std::memory_order_acquire)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kRowsMaxWarps * warp_bytes);
-    if (e != cudaSuccess) return (int)e;
-    asked[dev].store(true, std::memory_order_release);
-  }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((p.F + ft - 1) / ft, 1, 1);

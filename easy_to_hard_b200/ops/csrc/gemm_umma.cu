@@ -569,13 +569,9 @@ static int launch(const E2hGemmParams& p, const CUtensorMap& ta, const CUtensorM
                       xchg_bytes(BN, p.splitk, DUAL, TF);
   if (smem > 227 * 1024) return -12;
   auto kern = umma_gemm_kernel<BN, DUAL, TF, EPI>;
-  static size_t configured = 0;  // per instantiation
-  if (smem > configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = smem;
-  }
+  static SmemAsk ask;  // per instantiation
+  const cudaError_t e = ask(kern, smem);
+  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   const int t_tiles = p.n_groups > 0 ? p.n_groups * ((p.group_tmax + BN - 1) / BN)

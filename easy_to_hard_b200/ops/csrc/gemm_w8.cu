@@ -571,13 +571,9 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   size_t smem = (size_t)fixed + (size_t)stages * STAGE;
   if (smem < 120 * 1024) smem = 120 * 1024;
   auto kern = umma_gemm_w8_kernel<BN, DUAL, QB>;
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = smem;
-  }
+  static SmemAsk ask;
+  const cudaError_t e = ask(kern, smem);
+  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((p.F + p.th - 1) / p.th, (p.T + BN - 1) / BN, p.splitk);

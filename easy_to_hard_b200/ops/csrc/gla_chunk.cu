@@ -27,7 +27,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
-#include <mutex>
 
 #include "flash_common.cuh"
 #include "gla.cuh"
@@ -603,12 +602,8 @@ static int scan_launch(const E2hGlaParams& p, cudaStream_t stream) {
                    (long long)p.n * p.ld, p.ld, p.vdim, kC);
   if (r) return r;
   const size_t smem = 1024 + 3072 + (size_t)kGsStages * (4 * NH + 4) * 64 * 128;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(gla_chunk_scan_kernel<NH>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(gla_chunk_scan_kernel<NH>, smem);
   if (err != cudaSuccess) return (int)err;
   const dim3 grid((p.vdim + 127) / 128, p.H, p.n_seg);
   return (int)launch(gla_chunk_scan_kernel<NH>, grid, dim3(kGsThreads), smem, stream, tq, tk, ta,
@@ -633,12 +628,8 @@ extern "C" int e2h_gla_chunk(const E2hGlaParams* pp, void* stream_v) {
   if (2LL * p.chunks * p.H * kC > 0x7fffffffLL) return -4;
   const int smem = prep_smem_bytes(p.dim, p.r);
   if (smem > 200 * 1024 || p.r > 128) return -5;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [] {
-    err = cudaFuncSetAttribute(gla_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               200 * 1024);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(gla_chunk_prep_kernel, 200 * 1024);
   if (err != cudaSuccess) return (int)err;
   int r = (int)launch(gla_chunk_prep_kernel, dim3((p.seg_max + kC - 1) / kC, p.H, p.n_seg),
                       dim3(kPrepThreads), (size_t)smem, stream, p);

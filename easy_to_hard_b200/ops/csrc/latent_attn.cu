@@ -30,7 +30,6 @@
 #include <float.h>
 #include <stdint.h>
 #include <string.h>
-#include <mutex>
 
 #include "flash_common.cuh"
 #include "launch.cuh"
@@ -724,11 +723,8 @@ static int latent_mma_launch(const LatentParams& p, cudaStream_t stream) {
   const int r = latent_map(&tm, p.cache, kd, rows, kd % 64 == 0);
   if (r) return r;
   auto kern = latent_attn_mma_kernel<MT, KQ, NP, FUSED>;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(kern, kMmaSmem);
   if (err != cudaSuccess) return (int)err;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -769,11 +765,8 @@ static int latent_any_launch(const LatentParams& p, cudaStream_t stream) {
   const size_t smem = sizeof(float) * (kLatHeads * kd + kLatKeys * (kd + 4));
   if (smem > 200 * 1024) return -2;
   auto kern = latent_attn_kernel<T, NC>;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(kern, 200 * 1024);
   if (err != cudaSuccess) return (int)err;
   return (int)launch(kern, dim3((p.H + kLatHeads - 1) / kLatHeads, p.n), dim3(kLatHeads * 32), smem,
                      stream, p);

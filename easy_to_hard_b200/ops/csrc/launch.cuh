@@ -9,8 +9,32 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <string.h>
+#include <mutex>
 
 namespace e2h {
+
+// More than 48 KB of dynamic shared memory has to be asked for once per kernel and device; one static
+// object per kernel remembers what each device has granted.
+class SmemAsk {
+ public:
+  template <typename Kernel>
+  cudaError_t operator()(Kernel* kernel, size_t bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const std::lock_guard<std::mutex> lock(mu_);
+    const bool known = dev >= 0 && dev < kDevices;
+    if (known && granted_[dev] >= bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && known) granted_[dev] = bytes;
+    return e;
+  }
+
+ private:
+  static constexpr int kDevices = 64;
+  std::mutex mu_;
+  size_t granted_[kDevices] = {};
+};
 
 inline int g_pdl = 0;
 

@@ -27,7 +27,6 @@
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
-#include <mutex>
 
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -334,18 +333,9 @@ extern "C" int e2h_sample(const float* logits, long long ld, int B, int vocab, f
   const size_t row_bytes = ((size_t)vocab * 4 + 15) / 16 * 16;
   const int in_smem = row_bytes <= (size_t)kSampMaxSmemRow ? 1 : 0;
   if (in_smem) {
-    static std::mutex mu;
-    static bool asked[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static SmemAsk ask;
+    const cudaError_t e = ask(sample_kernel, kSampMaxSmemRow);
     if (e != cudaSuccess) return (int)e;
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev >= 0 && dev < 64 && !asked[dev]) {
-      e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kSampMaxSmemRow);
-      if (e != cudaSuccess) return (int)e;
-      asked[dev] = true;
-    }
   }
   return (int)launch(sample_kernel, dim3(B), dim3(kSampThreads), in_smem ? row_bytes : 0,
                      (cudaStream_t)stream, logits, ld, vocab, temperature, top_k, seed, pos_ptr,

@@ -15,7 +15,6 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <mutex>
 
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -150,11 +149,8 @@ static int stream_norm_launch(const StreamNormParams& p, int n, cudaStream_t str
   const size_t smem = (size_t)p.W * 4;
   if (smem > 200 * 1024) return -2;
   auto kern = stream_norm_kernel<T>;
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
+  static SmemAsk ask;
+  const cudaError_t err = ask(kern, 200 * 1024);
   if (err != cudaSuccess) return (int)err;
   const int per = (p.W + 3) / 4;
   const int threads = per >= 512 ? 512 : per >= 256 ? 256 : 128;

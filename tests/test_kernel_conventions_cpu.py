@@ -37,3 +37,15 @@ def test_every_kernel_given_to_the_pdl_launch_helper_waits_for_its_predecessor()
             assert "pdl_wait_prior()" in bodies[name], f"{src.name}: {name}"
             checked += 1
     assert checked >= 8
+
+
+def test_shared_memory_is_asked_for_on_every_device():
+    """cudaFuncSetAttribute holds for the current device only: what remembers an earlier call per process
+    fails on a second GPU. SmemAsk (launch.cuh) remembers it per device, one static object per kernel."""
+    for src in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        if src.name == "launch.cuh":
+            continue
+        text = src.read_text()
+        assert "cudaFuncSetAttribute" not in text, src.name
+        asks = re.findall(r"\b(?:ask|ask_\w+)\((\w+(?:<[^;]*?>)?),", text)
+        assert len(asks) >= len(re.findall(r"static SmemAsk", text)), src.name
