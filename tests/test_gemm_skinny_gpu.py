@@ -81,3 +81,31 @@ def test_rope_and_cache(T, pos, H, G, D, K):
     for a, b in zip(*outs):        # two bf16 roundings of sums in another order
         assert bool(((a - b).abs() <= 2.0 ** -6 * b.abs() + 2.0 ** -7).all())
     assert bool((outs[0][1] == 0).all()) == (pos >= S)
+
+
+@pytest.mark.parametrize("H,G,D,K", [(32, 32, 128, 256), (64, 8, 128, 192), (8, 2, 64, 264)])
+@pytest.mark.parametrize("T,pos", [(17, 0), (64, 39), (128, 7)])
+def test_rope_and_cache_against_the_rotation(T, pos, H, G, D, K):
+    """The fp32 sum and its rotation may each differ by one bf16 step, of the larger of the pair."""
+    from easy_to_hard_b200.ops import gemm, reference
+    S = 40
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn((H + 2 * G) * D, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    freqs = reference.precompute_freqs_cis(S, D, 10000.0, dtype=torch.bfloat16, device="cuda")
+    at = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    q = torch.zeros(T, H * D, device="cuda").bfloat16()
+    kc, vc = (torch.zeros(T, G, S, D, device="cuda").bfloat16() for _ in range(2))
+    gemm.linear_qkv_rope(x, w, q, freqs=freqs, pos_base=at, sq=1, n_head=H, n_kv=G, head_dim=D,
+                         kcache=kc, vcache=vc)
+    _status_ok()
+    raw = (x.double() @ w.double().t()).to(torch.bfloat16).view(T, 1, H + 2 * G, D)
+    f = freqs[pos:pos + 1]
+    wants = (reference.apply_rotary_emb(raw[:, :, :H], f), reference.apply_rotary_emb(raw[:, :, H:H + G], f),
+             raw[:, :, H + G:])
+    for got, want in zip((q.view(T, H, D), kc[:, :, pos], vc[:, :, pos]), wants):
+        want = want[:, 0].float()
+        assert bool(((got.float() - want).abs() <= 2.0 ** -6 * want.abs().max()).all())
+        assert float((got.float() - want).norm()) <= 2.0 ** -8 * float(want.norm())
+    other = torch.arange(S, device="cuda") != pos
+    assert not kc[:, :, other].any() and not vc[:, :, other].any()
