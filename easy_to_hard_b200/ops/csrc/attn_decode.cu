@@ -207,6 +207,7 @@ __device__ __noinline__ void attn_run_plain(const __nv_bfloat16* q, const __nv_b
 }
 
 // D = 16 * 8 * R : each lane of the half-warp holds R groups of 8 consecutive elements.
+// (three CTAs per SM leave the mma form 128 registers, at which it spills 24 bytes)
 template <int D, int G>
 __global__ void __launch_bounds__(kAttnThreads, AttnForm<D, G>::mma ? 3 : 0)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kcache,
@@ -437,130 +438,130 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
           *reinterpret_cast<float2*>(&sm_acc[warp][g][8 * i + 2 * t]) = make_float2(o[i][0], o[i][1]);
       }
     } else {
-    float qv[G][R][8];
+      float qv[G][R][8];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const int h = w.hk * G + g;
+      for (int g = 0; g < G; ++g) {
+        const int h = w.hk * G + g;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (lane_active) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(
-              q + ((long long)w.b * n_head + h) * D + (r * LPK + hl) * 8);
-          unpack8(raw, qv[g][r]);
+        for (int r = 0; r < R; ++r) {
+          if (lane_active) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(
+                q + ((long long)w.b * n_head + h) * D + (r * LPK + hl) * 8);
+            unpack8(raw, qv[g][r]);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) qv[g][r][i] *= scale;
-        } else {
+            for (int i = 0; i < 8; ++i) qv[g][r][i] *= scale;
+          } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) qv[g][r][i] = 0.f;
-        }
-      }
-    }
-    float m[G], l[G], acc[G][R][8];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      m[g] = -FLT_MAX;
-      l[g] = 0.f;
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[g][r][i] = 0.f;
-    }
-
-    for (int c = 0; c < n_here; ++c) {
-      if (!dead && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag, status, kStatusTimeoutFull))
-        dead = true;
-      if (!dead) {
-        const int j0 = w.start + (w.ch + c) * kChunk;
-        const uint8_t* ks = attn_smem + s * 2 * kTileBytes;
-        const uint8_t* vs = ks + kTileBytes;
-        uint4 kr[kKeysPerIter][R], vr[kKeysPerIter][R];
-#pragma unroll
-        for (int u = 0; u < kKeysPerIter; ++u) {
-          const int row = u * kSlots + slot;
-          const bool ok = j0 + row <= pos && lane_active;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int o = (row * D + (r * LPK + hl) * 8) * 2;
-            kr[u][r] = ok ? *reinterpret_cast<const uint4*>(ks + o) : make_uint4(0, 0, 0, 0);
-            vr[u][r] = ok ? *reinterpret_cast<const uint4*>(vs + o) : make_uint4(0, 0, 0, 0);
-          }
-        }
-        // the values are in registers: the stage can be refilled while they are used
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
-        // the four keys of this half-warp go through the running softmax together: one
-        // rescale of the accumulator per four keys instead of one per key (the kernel is close
-        // to instruction-issue bound: 63 % issue-active at 0.86 of the copy bandwidth)
-        float kf[kKeysPerIter][R][8];
-#pragma unroll
-        for (int u = 0; u < kKeysPerIter; ++u)
-#pragma unroll
-          for (int r = 0; r < R; ++r) unpack8(kr[u][r], kf[u][r]);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          float sc[kKeysPerIter];
-#pragma unroll
-          for (int u = 0; u < kKeysPerIter; ++u) {
-            float d = 0.f;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-              for (int i = 0; i < 8; ++i) d += qv[g][r][i] * kf[u][r][i];
-            sc[u] = d;
-          }
-          // reduce over the 16 lanes of the half-warp, the four keys interleaved
-#pragma unroll
-          for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < kKeysPerIter; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
-          float mn = m[g];
-#pragma unroll
-          for (int u = 0; u < kKeysPerIter; ++u)
-            if (j0 + u * kSlots + slot <= pos) mn = fmaxf(mn, sc[u]);
-          const float corr = __expf(m[g] - mn);
-          float pj[kKeysPerIter], psum = 0.f;
-#pragma unroll
-          for (int u = 0; u < kKeysPerIter; ++u) {
-            pj[u] = (j0 + u * kSlots + slot <= pos) ? __expf(sc[u] - mn) : 0.f;
-            psum += pj[u];
-          }
-          l[g] = l[g] * corr + psum;
-          m[g] = mn;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            float vf[kKeysPerIter][8];
-#pragma unroll
-            for (int u = 0; u < kKeysPerIter; ++u) unpack8(vr[u][r], vf[u]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float a = acc[g][r][i] * corr;
-#pragma unroll
-              for (int u = 0; u < kKeysPerIter; ++u) a += pj[u] * vf[u][i];
-              acc[g][r][i] = a;
-            }
+            for (int i = 0; i < 8; ++i) qv[g][r][i] = 0.f;
           }
         }
       }
-      if (++s == stages) {
-        s = 0;
-        ph ^= 1;
-      }
-    }
-
-    // ---- this (sequence, head) is done as far as this CTA goes: merge the 8 half-warp partials
+      float m[G], l[G], acc[G][R][8];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (hl == 0) {
-        sm_m[slot][g] = m[g];
-        sm_l[slot][g] = l[g];
-      }
-      if (lane_active) {
+      for (int g = 0; g < G; ++g) {
+        m[g] = -FLT_MAX;
+        l[g] = 0.f;
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sm_acc[slot][g][(r * LPK + hl) * 8 + i] = acc[g][r][i];
+          for (int i = 0; i < 8; ++i) acc[g][r][i] = 0.f;
       }
-    }
+
+      for (int c = 0; c < n_here; ++c) {
+        if (!dead && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag, status, kStatusTimeoutFull))
+          dead = true;
+        if (!dead) {
+          const int j0 = w.start + (w.ch + c) * kChunk;
+          const uint8_t* ks = attn_smem + s * 2 * kTileBytes;
+          const uint8_t* vs = ks + kTileBytes;
+          uint4 kr[kKeysPerIter][R], vr[kKeysPerIter][R];
+#pragma unroll
+          for (int u = 0; u < kKeysPerIter; ++u) {
+            const int row = u * kSlots + slot;
+            const bool ok = j0 + row <= pos && lane_active;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const int o = (row * D + (r * LPK + hl) * 8) * 2;
+              kr[u][r] = ok ? *reinterpret_cast<const uint4*>(ks + o) : make_uint4(0, 0, 0, 0);
+              vr[u][r] = ok ? *reinterpret_cast<const uint4*>(vs + o) : make_uint4(0, 0, 0, 0);
+            }
+          }
+          // the values are in registers: the stage can be refilled while they are used
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
+          // the four keys of this half-warp go through the running softmax together: one
+          // rescale of the accumulator per four keys instead of one per key (the kernel is close
+          // to instruction-issue bound: 63 % issue-active at 0.86 of the copy bandwidth)
+          float kf[kKeysPerIter][R][8];
+#pragma unroll
+          for (int u = 0; u < kKeysPerIter; ++u)
+#pragma unroll
+            for (int r = 0; r < R; ++r) unpack8(kr[u][r], kf[u][r]);
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            float sc[kKeysPerIter];
+#pragma unroll
+            for (int u = 0; u < kKeysPerIter; ++u) {
+              float d = 0.f;
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) d += qv[g][r][i] * kf[u][r][i];
+              sc[u] = d;
+            }
+            // reduce over the 16 lanes of the half-warp, the four keys interleaved
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+              for (int u = 0; u < kKeysPerIter; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
+            float mn = m[g];
+#pragma unroll
+            for (int u = 0; u < kKeysPerIter; ++u)
+              if (j0 + u * kSlots + slot <= pos) mn = fmaxf(mn, sc[u]);
+            const float corr = __expf(m[g] - mn);
+            float pj[kKeysPerIter], psum = 0.f;
+#pragma unroll
+            for (int u = 0; u < kKeysPerIter; ++u) {
+              pj[u] = (j0 + u * kSlots + slot <= pos) ? __expf(sc[u] - mn) : 0.f;
+              psum += pj[u];
+            }
+            l[g] = l[g] * corr + psum;
+            m[g] = mn;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              float vf[kKeysPerIter][8];
+#pragma unroll
+              for (int u = 0; u < kKeysPerIter; ++u) unpack8(vr[u][r], vf[u]);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                float a = acc[g][r][i] * corr;
+#pragma unroll
+                for (int u = 0; u < kKeysPerIter; ++u) a += pj[u] * vf[u][i];
+                acc[g][r][i] = a;
+              }
+            }
+          }
+        }
+        if (++s == stages) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+
+      // ---- this (sequence, head) is done as far as this CTA goes: merge the 8 half-warp partials
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if (hl == 0) {
+          sm_m[slot][g] = m[g];
+          sm_l[slot][g] = l[g];
+        }
+        if (lane_active) {
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sm_acc[slot][g][(r * LPK + hl) * 8 + i] = acc[g][r][i];
+        }
+      }
     }
     consumers_sync();
     // which of the pair's CTAs this one is, and how many there are

@@ -559,17 +559,17 @@ umma_gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           if (DUAL || !rope) {
 #pragma unroll
-          for (int j = 0; j < kChunkTok; ++j) {
-            float y;
-            if constexpr (DUAL) {
-              const float g = bf16_round(v[j] * sc), u = bf16_round(v2[j] * sc2);
-              y = bf16_round(silu(g)) * u;
-            } else {
-              y = v[j] * sc;
-              if (with_res) y = bf16_round(y) + __bfloat162float(sr[j * 128 + lane_row]);
+            for (int j = 0; j < kChunkTok; ++j) {
+              float y;
+              if constexpr (DUAL) {
+                const float g = bf16_round(v[j] * sc), u = bf16_round(v2[j] * sc2);
+                y = bf16_round(silu(g)) * u;
+              } else {
+                y = v[j] * sc;
+                if (with_res) y = bf16_round(y) + __bfloat162float(sr[j * 128 + lane_row]);
+              }
+              so[j * 128 + lane_row] = __float2bfloat16_rn(y);
             }
-            so[j * 128 + lane_row] = __float2bfloat16_rn(y);
-          }
           }
           fence_proxy_async_smem();
           epi_bar_sync();

@@ -18,15 +18,15 @@
 //     registers held 22016 x 4096 int8 weights to 25 us where this takes 21), and no barrier is
 //     needed. The first ring is filled before the wait for the preceding kernel (weights are never
 //     written by a predecessor of a PDL chain);
-//   * activations come through L1 and L2 the same way, T rows of them for every tile: they are what
-//     int4 at 16 rows waits for, besides the five instructions a pair of its codes takes to expand.
+//   * activations come through L1 and L2 the same way, T rows of them for every tile: from 9 rows on
+//     they are what long sums wait for (rows_pays in ops/gemm.py).
 //
 // Time per launch in a chain of launches with distinct weights (L2 cold), tcgen05 kernel -> this one:
 //                                     bf16, 1 row     bf16, 16 rows   int8, 8 rows    int4, 8 rows
-//   12288 x 4096                      33.8 -> 21.3    26.2 -> 21.9    30.0 -> 15.6    29.7 -> 14.6 us
-//   4096 x 4096 + residual            12.6 ->  7.4    12.7 -> 10.1    13.5 ->  7.8    13.6 ->  7.5
-//   2 x 11008 x 4096, gated           47.4 -> 30.4    42.7 -> 36.0    50.6 -> 22.4    49.9 -> 20.7
-//   4096 x 11008 + residual           21.9 -> 16.4    21.8 -> 21.8    22.9 -> 13.7    22.5 -> 14.6
+//   12288 x 4096                      33.8 -> 21.3    26.2 -> 22.4    30.0 -> 15.6    29.7 -> 14.6 us
+//   4096 x 4096 + residual            12.6 ->  7.4    12.7 -> 10.3    13.5 ->  7.8    13.6 ->  7.5
+//   2 x 11008 x 4096, gated           47.4 -> 30.4    42.7 -> 35.7    50.6 -> 22.4    49.9 -> 20.7
+//   4096 x 11008 + residual           21.9 -> 16.4    (not taken)     22.9 -> 13.7    22.5 -> 14.6
 //   256 x 256                          6.0 ->  1.8
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -83,6 +83,8 @@ __host__ __device__ inline int xchg_bytes(int bn, int splitk, int dual, int tf) 
   return (splitk - 1) * (bn / splitk) * tf * 4 * (dual ? 2 : 1);
 }
 
+// (two CTAs per SM leave a compiled-in kernel 96 registers: the gated ones spill 16 to 28 bytes, outside
+// the k-loop)
 template <int BN, bool DUAL, int TF, int EPI>
 __global__ void __launch_bounds__(kThreads, EPI >= 0 ? 2 : 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,

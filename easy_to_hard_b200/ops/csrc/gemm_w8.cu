@@ -44,7 +44,7 @@ constexpr int kW8Threads = 320;     // TMA warp, MMA warp, 8 converter warps (4 
 constexpr int kW8MaxStages = 8;
 constexpr int kW8Ctrl = 1024;
 constexpr int kW8Kps = 2;          // 64-wide k-blocks per pipeline stage
-constexpr int kW8ConvMax = 4;      // converted-tile buffers: 4 (3 for a dual GEMM, whose tiles are twice as large)
+constexpr int kW8ConvMax = 4;      // converted-tile buffers: 4 (3 for a dual GEMM: twice as large)
 constexpr int kW8ACol0 = 128;      // tensor-memory column of the first converted-tile buffer
 constexpr int kW8ACols = 64;       // columns of one converted [128 x 128 k] bf16 tile
 constexpr int kW8TmemCols = 512;
@@ -197,7 +197,8 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // The whole warp walks the loop and one lane issues: the operands of an instruction are then
     // uniform values. In a branch of a single lane an instruction took 66 to 88 cycles to issue (64
     // rows) where the tensor core takes 32. Chain of launches, 12288 x 4096 int8, 64 rows: 30.0 -> 27 us.
-    // What is left is the converters' instruction issue.
+    // What is left is the converters' chain: a warp loads, converts, stores, waits for the store and
+    // arrives, one stage after the other (their instructions are a quarter of a stage's cycles).
     const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, BN, 0, 0);
     // descriptors: constant high word, base low words once, one add per instruction; stage and
