@@ -18,12 +18,13 @@
 // 16-byte pieces of a small vocabulary (elements, where a group would go without) go to different
 // groups, so that no group is empty or much smaller than another: with neighbours in one group,
 // fewer groups than top_k had entries, and every entry became a candidate (2000 logits, top 200: 151
-// us, 11 now). Otherwise, or if more than 1024 entries reach the bound (many equal logits, top_k
-// near 256; ranking 1400 candidates takes 77 to 150 us, the passes 44 over 32000 logits): a 4-pass,
-// 8-bit radix select over the order-preserving integer image of the fp32 logits. The row (128 KB at a 32k
-// vocabulary) is copied into shared memory once and all five passes read it from there: the passes
-// are chains of dependent loads (a warp-wide match between them), which from L2 cost ~13 us per pass
-// and ~100 us per step; rows that do not fit stay in global memory.
+// us, 11 now). Otherwise, or if more than 1024 entries (512 of a small vocabulary) reach the bound (many
+// equal logits, top_k near 256; ranking 1400 candidates takes 77 to 150 us and 1000 take 43, the
+// passes 44 over 32000 logits and 12 over 4000): a 4-pass, 8-bit radix select over the
+// order-preserving integer image of the fp32 logits. The row (128 KB at a 32k vocabulary) is copied
+// into shared memory once and all five passes read it from there: the passes are chains of dependent
+// loads (a warp-wide match between them), which from L2 cost ~13 us per pass and ~100 us per step; rows
+// that do not fit stay in global memory.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -170,7 +171,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int vocab, float t
     for (int i = (vocab & ~3) + threadIdx.x; i < vocab; i += kSampThreads) collect(srow[i], i);
     __syncthreads();
     const int n = n_cand;
-    if (n <= kSampCandMax) {
+    if (n <= (spread ? kSampCandMax / 2 : kSampCandMax)) {
       // the k-th largest key: the candidate with fewer than k keys above it and at least k at
       // or above it (all such candidates carry the same key)
       for (int c = threadIdx.x; c < n; c += blockDim.x) {

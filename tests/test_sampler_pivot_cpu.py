@@ -45,7 +45,7 @@ def test_candidate_pivot_is_the_kth_largest(seed, k):
     assert pivot == np.sort(row)[-k]
     assert n_cand >= k
     if seed % 3 and k < 256:
-        assert n_cand <= 1024               # the list the kernel keeps is long enough
+        assert n_cand <= (512 if v < 16 * THREADS else 1024)    # short enough to be ranked
 
 
 @pytest.mark.parametrize("v", [500, 1000, 1024, 2000, 4000, 4096, 5003])
