@@ -375,12 +375,15 @@ static int launch_parts_rows(const void* h_in, const PartPtrs& parts, int n_part
 // One CTA per row, one 16-byte vector per thread, so a row is one load, one block sum and one
 // store; the weight vector is fetched before the wait for the predecessor kernel (weights are
 // never written inside a programmatic-dependent-launch chain). Same arithmetic as
-// rmsnorm_fwd_kernel: x = bf16(bf16(h * rstd) * w).
+// rmsnorm_fwd_kernel: x = bf16(bf16(h * rstd) * w). With `tokens` the row is a token's embedding.
 __global__ void rmsnorm_row_latency_kernel(const __nv_bfloat16* __restrict__ h_in,
                                            const __nv_bfloat16* __restrict__ weight,
                                            __nv_bfloat16* __restrict__ h_out,
                                            __nv_bfloat16* __restrict__ x_out,
-                                           float* __restrict__ rstd_out, int dim, float eps) {
+                                           float* __restrict__ rstd_out, int dim, float eps,
+                                           const int* __restrict__ tokens,
+                                           const __nv_bfloat16* __restrict__ emb, int emb_rows,
+                                           int* status) {
   __shared__ float red[32];
   const int i = threadIdx.x * 8;
   const bool on = i < dim;
@@ -389,10 +392,12 @@ __global__ void rmsnorm_row_latency_kernel(const __nv_bfloat16* __restrict__ h_i
   pdl_launch_dependents();
   pdl_wait_prior();
   const long long base = (long long)blockIdx.x * dim;
+  const __nv_bfloat16* src =
+      tokens ? emb_row(tokens, blockIdx.x, emb, emb_rows, dim, status) : h_in + base;
   float v[8], w[8];
   float ss = 0.f;
   if (on) {
-    const BF8 hv = *reinterpret_cast<const BF8*>(h_in + base + i);
+    const BF8 hv = src ? *reinterpret_cast<const BF8*>(src + i) : BF8{};
     unpack8(hv, v);
     unpack8(wv, w);
 #pragma unroll
@@ -429,34 +434,40 @@ int e2h_rmsnorm_fwd(const void* h_in, const int* tokens, const void* emb, int em
                                      eps, flags, use_count, ticket, status, stream);
     if (rc != -100) return rc;
   }
+  const bool plain = n_part == 0 && x_out != nullptr && flags == nullptr && dim % 8 == 0 &&
+                     aligned16(x_out) && aligned16(weight) &&
+                     (tokens ? aligned16(emb) : h_in != nullptr && aligned16(h_in)) &&
+                     (h_out == nullptr || aligned16(h_out));
   // plain row normalisation of many tokens: the vectorised streaming kernel
-  if (T >= 256 && h_in != nullptr && tokens == nullptr && n_part == 0 && h_out == nullptr &&
-      x_out != nullptr && flags == nullptr && dim % 8 == 0 && dim <= 8192 && aligned16(h_in) &&
-      aligned16(x_out) && aligned16(weight)) {
+  if (T >= 256 && plain && dim <= 8192 && (tokens != nullptr) == (h_out != nullptr)) {
     const int threads = dim > 4096 ? 256 : 128;
     const int nv = (dim / 8 + threads - 1) / threads;
     cudaStream_t st = (cudaStream_t)stream;
-#define E2H_GO(NV)                                                                            \
-  rmsnorm_rows_kernel<NV><<<T, threads, 0, st>>>((const __nv_bfloat16*)h_in,                  \
-                                                 (const __nv_bfloat16*)weight,                \
-                                                 (__nv_bfloat16*)x_out, rstd_out, dim, eps)
-    if (nv <= 1) E2H_GO(1); else if (nv == 2) E2H_GO(2); else if (nv <= 4) E2H_GO(4);
+#define E2H_GO(NV, EMB)                                                                         \
+  rmsnorm_rows_kernel<NV, EMB><<<resident_blocks(rmsnorm_rows_kernel<NV, EMB>, threads, T),     \
+                                 threads, 0, st>>>(                                             \
+      (const __nv_bfloat16*)(EMB ? emb : h_in), (const __nv_bfloat16*)weight,                   \
+      (__nv_bfloat16*)x_out, rstd_out, T, dim, eps, tokens, emb_rows, (__nv_bfloat16*)h_out, status)
+    if (tokens) {
+      if (nv <= 1) E2H_GO(1, true); else if (nv == 2) E2H_GO(2, true); else E2H_GO(4, true);
+    } else {
+      if (nv <= 1) E2H_GO(1, false); else if (nv == 2) E2H_GO(2, false); else E2H_GO(4, false);
+    }
 #undef E2H_GO
-    if (nv <= 4) return (int)cudaGetLastError();
+    return (int)cudaGetLastError();
   }
   // a few rows (decode): the latency-oriented kernel, one 16-byte vector per thread
   static const bool latency_form = [] {   // E2H_NORM_LATENCY=0: measurement switch
     const char* e = getenv("E2H_NORM_LATENCY");
     return !(e && e[0] == '0');
   }();
-  if (latency_form && T < 256 && h_in != nullptr && tokens == nullptr && n_part == 0 &&
-      x_out != nullptr && flags == nullptr && dim % 8 == 0 && dim / 8 <= 1024 && aligned16(h_in) &&
-      aligned16(x_out) && aligned16(weight) && (h_out == nullptr || aligned16(h_out))) {
+  if (latency_form && T < 256 && plain && dim / 8 <= 1024) {
     const int threads_l = (dim / 8 + 31) / 32 * 32;
     return (int)launch(rmsnorm_row_latency_kernel, dim3(T), dim3(threads_l), 0,
                        (cudaStream_t)stream, (const __nv_bfloat16*)h_in,
                        (const __nv_bfloat16*)weight, (__nv_bfloat16*)h_out,
-                       (__nv_bfloat16*)x_out, rstd_out, dim, eps);
+                       (__nv_bfloat16*)x_out, rstd_out, dim, eps, tokens, (const __nv_bfloat16*)emb,
+                       emb_rows, status);
   }
   const int threads = dim >= 2048 ? 512 : 128;
   const size_t smem = (dim + 32) * sizeof(float);
@@ -491,9 +502,10 @@ int e2h_rmsnorm_bwd(const void* x, const void* dy, const void* weight, const voi
     const int nv = (dim / 8 + threads - 1) / threads;
     cudaStream_t st = (cudaStream_t)stream;
 #define E2H_GO(NV)                                                                           \
-  rmsnorm_bwd_rows_kernel<NV><<<T, threads, 0, st>>>(                                        \
+  rmsnorm_bwd_rows_kernel<NV><<<resident_blocks(rmsnorm_bwd_rows_kernel<NV>, threads, T),    \
+                                threads, 0, st>>>(                                           \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)weight,       \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dim, eps)
+      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, T, dim, eps)
     if (nv <= 1) E2H_GO(1); else if (nv == 2) E2H_GO(2); else if (nv <= 4) E2H_GO(4);
 #undef E2H_GO
     if (nv <= 4) return (int)cudaGetLastError();
