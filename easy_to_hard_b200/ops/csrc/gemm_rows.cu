@@ -42,7 +42,6 @@
 namespace e2h {
 
 constexpr int kRowsMaxWarps = 8;
-constexpr int kRowsRingBytes = 12 * 1024;    // per warp: 16 warps of an SM have 192 KB of ring
 
 // 16 (or 4) bytes from global to shared memory, zeros where `in` is false; nothing is read then.
 __device__ __forceinline__ void cp_async16_once(uint32_t dst, const void* src, bool in, uint64_t policy) {
@@ -82,25 +81,26 @@ struct RowsUnit {
 };
 
 // Shared memory of one warp: a ring of S stages of UN units, a unit being the lane-major vectors
-// [MT][2] of A, [NT][b_vec] of B and, for int4, [MT][2] (scale, zero) pairs.
-template <int QB, int MT, int NT>
+// [MT][2] of A, [NT][b_vec] of B and, for int4, [MT][2] (scale, zero) pairs. RB bytes of it at most: 12 KB,
+// with which 16 warps share an SM, or 8 KB for 24.
+template <int QB, int MT, int NT, int RB>
 struct RowsRing {
   using U = RowsUnit<QB>;
   static constexpr int a_bytes = MT * 2 * 512, b_bytes = NT * U::b_vec * 512;
   static constexpr int unit_bytes = a_bytes + b_bytes + (QB == 4 ? MT * 2 * 128 : 0);
-  static constexpr int UN = QB == 16 && MT == 1 ? 2 : 1;
+  static constexpr int UN = QB == 16 && MT == 1 && RB > 8192 ? 2 : 1;
   static constexpr int stage_bytes = UN * unit_bytes;
-  static constexpr int want = kRowsRingBytes / stage_bytes;
+  static constexpr int want = RB / stage_bytes;
   static constexpr int S = want < 2 ? 2 : want > 8 ? 8 : want;
   static constexpr int bytes = S * stage_bytes;
 };
 
 // QB: bits per weight. MT: 16-row tiles of a warp (a gated product: tile 0 of A above tile 0 of A2).
-// NT: groups of 8 rows of B.
-template <int QB, int MT, int NT, bool DUAL>
+// NT: groups of 8 rows of B. SHARE: CTAs take equal shares instead of whole tiles.
+template <int QB, int MT, int NT, bool DUAL, int RB, bool SHARE>
 __global__ void __launch_bounds__(kRowsMaxWarps * 32, 2) gemm_rows_kernel(const E2hGemmParams p) {
   using U = RowsUnit<QB>;
-  using R = RowsRing<QB, MT, NT>;
+  using R = RowsRing<QB, MT, NT, RB>;
   static_assert(!DUAL || MT == 2, "a gated product pairs two tiles");
   constexpr int FT = DUAL ? 16 : 16 * MT;      // output features of a CTA
   constexpr int PITCH = 8 * NT + 4;            // floats per feature in the exchange buffer
@@ -109,17 +109,25 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, 2) gemm_rows_kernel(const 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int g = lane >> 2, t4 = lane & 3;
-  const int f0 = blockIdx.x * FT;
+  // this CTA's features: a tile, or an equal share of at most as many, in pairs (the rotation turns pairs)
+  int f0 = blockIdx.x * FT, f1 = f0 + FT;
+  if constexpr (SHARE) {
+    const long long pairs = (p.F + 1) / 2;
+    f0 = 2 * (int)(blockIdx.x * pairs / gridDim.x);
+    f1 = min(2 * (int)((blockIdx.x + 1) * pairs / gridDim.x), p.F);
+  }
   pdl_launch_dependents();
 
-  // this lane's rows (clamped: rows past the end repeat the last one and are masked at the end)
+  // this lane's rows (one past the share is not loaded, and masked at the end)
   const uint8_t* arow[MT][2];
   int frow[MT][2];
+  bool own[MT][2];
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int f = min(f0 + (DUAL ? 0 : 16 * m) + g + 8 * r, p.F - 1);
+      const int at = f0 + (DUAL ? 0 : 16 * m) + g + 8 * r, f = min(at, p.F - 1);
+      own[m][r] = !SHARE || at < f1;
       const void* base = (DUAL && m == 1) ? p.a2 : p.a;
       const long long ld = (DUAL && m == 1) ? p.lda2 : p.lda;   // bf16: elements, else bytes
       frow[m][r] = f;
@@ -149,8 +157,9 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, 2) gemm_rows_kernel(const 
       for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
+          const bool mine = in && own[m][r];
           cp_async16_once(ring_a + dst + (m * 2 + r) * 512,
-                          in ? arow[m][r] + (long long)(u + i) * 64 : arow[m][r], in, once);
+                          mine ? arow[m][r] + (long long)(u + i) * 64 : arow[m][r], mine, once);
           if constexpr (QB == 4) {
             const __nv_bfloat162* z =
                 static_cast<const __nv_bfloat162*>((DUAL && m == 1) ? p.qsz2 : p.qsz);
@@ -272,7 +281,7 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, 2) gemm_rows_kernel(const 
   if (warp >= NT || 8 * warp >= p.T) return;
 
   // epilogue: warp n finishes tokens 8 n .. 8 n + 7, a lane owns a feature
-  const bool lane_ok = lane < FT;
+  const bool lane_ok = lane < f1 - f0;
   const int row = lane_ok ? lane : 0;
   float v[8], v2[DUAL ? 8 : 1];
 #pragma unroll
@@ -296,17 +305,16 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, 2) gemm_rows_kernel(const 
   epilogue8<DUAL>(p, lane_ok ? f0 + lane : p.F, 8 * warp, v, v2, p.T);
 }
 
-template <int QB, int MT, int NT, bool DUAL>
-static int rows_launch(const E2hGemmParams& p, int warps, cudaStream_t stream) {
-  const int ft = DUAL ? 16 : 16 * MT;
-  auto kern = gemm_rows_kernel<QB, MT, NT, DUAL>;
-  constexpr int warp_bytes = RowsRing<QB, MT, NT>::bytes;
+template <int QB, int MT, int NT, bool DUAL, int RB, bool SHARE>
+static int rows_launch(const E2hGemmParams& p, int ctas, int warps, cudaStream_t stream) {
+  auto kern = gemm_rows_kernel<QB, MT, NT, DUAL, RB, SHARE>;
+  constexpr int warp_bytes = RowsRing<QB, MT, NT, RB>::bytes;
   static SmemAsk ask;
   const cudaError_t e = ask(kern, kRowsMaxWarps * warp_bytes);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((p.F + ft - 1) / ft, 1, 1);
+  cfg.gridDim = dim3(ctas, 1, 1);
   cfg.blockDim = dim3(32 * warps, 1, 1);
   cfg.dynamicSmemBytes = (size_t)warps * warp_bytes;
   cfg.stream = stream;
@@ -321,10 +329,19 @@ static int rows_launch(const E2hGemmParams& p, int warps, cudaStream_t stream) {
 }
 
 template <int QB, int NT>
-static int rows_dispatch(const E2hGemmParams& p, int mt, int warps, cudaStream_t stream) {
-  if (p.dual) return rows_launch<QB, 2, NT, true>(p, warps, stream);
-  if (mt == 2) return rows_launch<QB, 2, NT, false>(p, warps, stream);
-  return rows_launch<QB, 1, NT, false>(p, warps, stream);
+static int rows_dispatch(const E2hGemmParams& p, int mt, int ctas, int warps, bool share,
+                         bool short_ring, cudaStream_t stream) {
+  if (p.dual) return rows_launch<QB, 2, NT, true, 12288, false>(p, ctas, warps, stream);
+  if constexpr (QB == 16 && NT == 1) {
+    if (short_ring && mt == 2) return rows_launch<QB, 2, NT, false, 8192, true>(p, ctas, warps, stream);
+    if (short_ring) return rows_launch<QB, 1, NT, false, 8192, true>(p, ctas, warps, stream);
+  }
+  if constexpr (QB == 8 || (QB == 16 && NT == 1)) {
+    if (share && mt == 2) return rows_launch<QB, 2, NT, false, 12288, true>(p, ctas, warps, stream);
+    if (share) return rows_launch<QB, 1, NT, false, 12288, true>(p, ctas, warps, stream);
+  }
+  if (mt == 2) return rows_launch<QB, 2, NT, false, 12288, false>(p, ctas, warps, stream);
+  return rows_launch<QB, 1, NT, false, 12288, false>(p, ctas, warps, stream);
 }
 
 }  // namespace e2h
@@ -368,11 +385,26 @@ extern "C" int e2h_gemm_rows(const E2hGemmParams* pp, int bits, void* stream_v) 
   const int mt = p.F >= 32 * 148 * (wide ? 1 : 2) ? 2 : 1;     // (rows_pays in ops/gemm.py knows this)
   const int ft = p.dual ? 16 : 16 * mt;
   const int tiles = (p.F + ft - 1) / ft;
-  int warps = tiles >= 148 * (p.T > 8 ? 2 : 4) ? 4 : 8;
+  // Three to six tiles a SM: as many CTAs there, with equal shares of the features. With whole tiles some SMs
+  // had one more than others, and with more CTAs than fit at once a last round ran half empty (12288
+  // features are 384 tiles on 296 places). bf16, up to 8 rows: three a SM fit at once with a ring of 8 KB, four
+  // make two rounds with 12 KB. Not for int4, whose time goes with the tiles' arithmetic, used rows or
+  // not (5120 x 13824, 8 rows 25.7 -> 38.8 us), nor for gated products; with one or two tiles, or seven and
+  // more, shares lost 3 to 5 %, as for bf16 from 9 rows on and for long sums in int8. us at 1 and 8 rows: 12288 x 4096 bf16 20.9 -> 17.3 and 22.1 -> 17.9, int8 14.7
+  // -> 13.2 and 15.3 -> 13.8 (16 rows 19.7 -> 15.8); 5120 x 5120 bf16 13.6 -> 10.7 and 14.6 -> 11.8, int8 11.1
+  // -> 10.1; 5760 x 2048 bf16 8.8 -> 6.7 and 9.8 -> 7.5.
+  const int per_sm = (tiles + 147) / 148;
+  const bool share = !p.dual && per_sm >= 3 && per_sm <= 6 &&
+                     (bits == 16 ? p.T <= 8 : bits == 8 && p.K <= 8192);
+  const int ctas = share ? 148 * per_sm : tiles;
+  const bool short_ring = share && bits == 16 && per_sm == 3;
+  int warps = tiles >= 148 * (p.T > 8 || share ? 2 : 4) ? 4 : 8;
+  if (short_ring || (share && bits == 16 && per_sm == 4 && p.K >= 4096)) warps = 8;
   while (warps > 2 && units < 2 * warps) warps >>= 1;    // (the epilogue of 16 rows takes two)
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-#define E2H_ROWS(QB_) \
-  return p.T <= 8 ? rows_dispatch<QB_, 1>(p, mt, warps, stream) : rows_dispatch<QB_, 2>(p, mt, warps, stream)
+#define E2H_ROWS(QB_)                                                                           \
+  return p.T <= 8 ? rows_dispatch<QB_, 1>(p, mt, ctas, warps, share, short_ring, stream)        \
+                  : rows_dispatch<QB_, 2>(p, mt, ctas, warps, share, short_ring, stream)
   if (bits == 16) E2H_ROWS(16);
   if (bits == 8) E2H_ROWS(8);
   E2H_ROWS(4);
