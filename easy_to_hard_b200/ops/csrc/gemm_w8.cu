@@ -6,15 +6,15 @@
 //   warp 0      TMA producer: per stage one int8 weight tile [128 features x 128 k] (128-byte rows,
 //               128B swizzle: the same row granularity as the bf16 GEMM) and the two matching bf16
 //               activation tiles [BN tokens x 64 k] (one 3-D box);
-//   warps 2-9   converters during the main loop (two threads per feature row, 64 k each):
-//               int8 -> bf16 two values per instruction -- a byte permute drops each byte into the
-//               mantissa of bf16(128) (0x4300 | low 7 bits), and one packed bf16 subtraction of
+//   warps 2-17  two groups of converters that take turns at the stages (two threads per feature row, 64
+//               k each): int8 -> bf16 two values per instruction -- a byte permute drops each byte
+//               into the mantissa of bf16(128) (0x4300 | low 7 bits), and one packed bf16 subtraction of
 //               128 or 256 (chosen by the sign bit) yields the exact integer. The converted row
 //               goes straight from registers into TENSOR memory (tcgen05.st, the thread's own
 //               lane, 32 columns = 64 k), where tcgen05.mma reads it as its A operand: the
 //               expanded tile never touches shared memory, whose bandwidth (16 KB read + 32 KB
 //               written + 32 KB read back per 128 k) held the earlier form at the bf16 rate.
-//               Several buffers alternate; afterwards the eight warps run the epilogue;
+//               Several buffers alternate; afterwards the first eight warps run the epilogue;
 //   warp 1      one thread issues tcgen05.mma (M = 128, N = BN, K = 16; A from tensor memory,
 //               the activation tile from shared memory) into the fp32 accumulator.
 //
@@ -40,7 +40,9 @@
 
 namespace e2h {
 
-constexpr int kW8Threads = 320;     // TMA warp, MMA warp, 8 converter warps (4 of them: epilogue)
+constexpr int w8_threads(int groups) {   // TMA warp, MMA warp, groups of 8 converter warps (the first: epilogue)
+  return 64 + 256 * groups;
+}
 constexpr int kW8MaxStages = 8;
 constexpr int kW8Ctrl = 1024;
 constexpr int kW8Kps = 2;          // 64-wide k-blocks per pipeline stage
@@ -67,8 +69,9 @@ __host__ __device__ inline int w8_xchg_bytes(int bn, int splitk, int dual) {
 
 // QB = 8: int8 weights with per-feature scales in the epilogue; QB = 4: packed int4 weights with
 // group-wise (scale, zero) pairs applied by the converters.
-template <int BN, bool DUAL, int QB>
-__global__ void __launch_bounds__(kW8Threads, 1)
+// GROUPS: converter groups that take turns at the stages.
+template <int BN, bool DUAL, int QB, int GROUPS>
+__global__ void __launch_bounds__(w8_threads(GROUPS), 1)
 umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                     const __grid_constant__ CUtensorMap tmB, const E2hGemmParams p) {
   constexpr int NMAT = DUAL ? 2 : 1;
@@ -197,8 +200,12 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // The whole warp walks the loop and one lane issues: the operands of an instruction are then
     // uniform values. In a branch of a single lane an instruction took 66 to 88 cycles to issue (64
     // rows) where the tensor core takes 32. Chain of launches, 12288 x 4096 int8, 64 rows: 30.0 -> 27 us.
-    // What is left is the converters' chain: a warp loads, converts, stores, waits for the store and
-    // arrives, one stage after the other (their instructions are a quarter of a stage's cycles).
+    // What bounds the kernel is the conversion: about 12 cycles of a scheduler's ALU per four int8 codes
+    // (quant_cvt.cuh). With one group of eight warps its loads, waits and hand-shakes came on top, a gated
+    // stage taking 1893 cycles of which 800 without the conversion; two groups overlap them. Chain of
+    // launches, 64 rows, one group and the older conversion -> now, int8 and int4 (us): 12288 x 4096 27.1 -> 21.9
+    // and 27.5 -> 22.9; gated 2 x 11008 x 4096 46.1 -> 37.4 and 48.9 -> 39.6; 4096 x 11008 20.8 -> 17.8 and 21.3
+    // -> 18.5; 4096 x 4096 12.2 -> 11.6. (16 warps on each stage were no faster than eight.)
     const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, BN, 0, 0);
     // descriptors: constant high word, base low words once, one add per instruction; stage and
@@ -248,9 +255,9 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 
   const bool is_conv = warp >= 2;
-  const bool is_epi = warp >= 2;
+  const bool is_epi = warp >= 2 && warp < 10;
   const int q = warp & 3;                             // tensor-memory lane quarter of this warp
-  const int half = (warp - 2) >> 2;                   // which of the quarter's two warps
+  const int half = ((warp - 2) >> 2) & 1;             // which of the quarter's two warps
   const int lane_row = q * 32 + lane;                 // feature row = tensor-memory lane
   const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
   if (is_conv) {
@@ -258,9 +265,12 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // thread (row, half): the 64 k of `row` that make up bf16 k-block `half` of the stage
     const int row = lane_row;
     const int sw = row & 7;                           // 128B-swizzle term of this row
+    const int group = (warp - 2) >> 3;                // of two, 0 takes the even stages, 1 the odd ones
     bool ok = true;
-    int s = 0;
-    uint32_t ph = 0;
+    int s = stages > 1 ? group : 0;
+    uint32_t ph = stages > 1 ? 0 : group;
+    int c = group;
+    uint32_t cph = 0;
     const int gshift = QB == 4 ? __ffs(p.groupsize) - 1 : 0;   // group size is a power of two
     // int4: the (scale, zero) pair of this row's group is a global load; the pair of the next
     // stage is fetched one iteration ahead so that its latency hides behind the barrier waits
@@ -279,17 +289,17 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
     };
-    load_sz(0);
-    for (int it = 0; it < n_it; ++it) {
-      const int c = it % kW8Conv;
+    load_sz(group);
+    for (int it = group; it < n_it; it += GROUPS) {
       __nv_bfloat162 sz_cur[NMAT];
 #pragma unroll
       for (int m = 0; m < NMAT; ++m) sz_cur[m] = sz_next[m];
-      load_sz(it + 1);
+      load_sz(it + GROUPS);
       const int s_cur = s;
       const uint32_t ph_cur = ph;
-      if (++s == stages) {
-        s = 0;
+      s += GROUPS;
+      while (s >= stages) {
+        s -= stages;
         ph ^= 1;
       }
       // every converter thread waits itself (one polling lane per warp plus a shuffle measured
@@ -297,8 +307,8 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       if (ok)
         ok = mbar_wait(smem_u32(&ctrl->full[s_cur]), ph_cur, abort_flag, p.status,
                        kStatusTimeoutFull) &&
-             mbar_wait(smem_u32(&ctrl->conv_empty[c]), ((it / kW8Conv) & 1) ^ 1, abort_flag,
-                       p.status, kStatusTimeoutEmpty);
+             mbar_wait(smem_u32(&ctrl->conv_empty[c]), cph ^ 1, abort_flag, p.status,
+                       kStatusTimeoutEmpty);
       tc_fence_after();
       if (ok) {
         const uint8_t* st = tiles + (size_t)s_cur * STAGE;
@@ -348,6 +358,11 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tc_fence_before();          // the stores are ordered before the arrival below
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->conv_full[c]));
+      c += GROUPS;
+      if (c >= kW8Conv) {
+        c -= kW8Conv;
+        cph ^= 1;
+      }
     }
   }
 
@@ -394,12 +409,13 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int c_begin = rank * slice;
     const bool lane_valid = lane_row < TH;
     const int f = lane_valid ? f0 + lane_row : p.F;   // rows past the tile are masked
-    // columns of this warp: with 64 or more, alternate groups of 32; with fewer, the first /
+    // columns of this warp: with 64 or more, alternate groups of W; with fewer, the first /
     // second half of the 8-column units
     const int units = slice >> 3;
+    constexpr int W = DUAL ? 16 : 32;    // columns per trip (two accumulators of 32 would not fit the registers)
     int c_first, c_last;
     if (units >= 8) {
-      c_first = 32 * half;
+      c_first = W * half;
       c_last = slice;
     } else {
       const int lo = units == 1 ? 1 : units >> 1;
@@ -408,12 +424,12 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     RopePre rope;
     if (staged && p.epi == E2H_EPI_ROPE_KV) rope = rope_prepare(p, f);
-    for (int c = c_first; c < c_last; c += 64) {
-      const int nb = (c_last - c) >= 32 ? 4 : (c_last - c) / 8;
-      float v[32], v2[DUAL ? 32 : 1];
+    for (int c = c_first; c < c_last; c += 2 * W) {
+      const int nb = (c_last - c) >= W ? W / 8 : (c_last - c) / 8;
+      float v[W], v2[DUAL ? W : 1];
       if (n_kb > 0) {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < W / 8; ++b) {
           if (b < nb) {
             tmem_ld_x8(taddr + c_begin + c + 8 * b, v + 8 * b);
             if constexpr (DUAL) tmem_ld_x8(taddr + BN + c_begin + c + 8 * b, v2 + 8 * b);
@@ -422,13 +438,13 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         tmem_ld_wait();
       } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < W; ++j) {
           v[j] = 0.f;
           if constexpr (DUAL) v2[j] = 0.f;
         }
       }
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
+      for (int b = 0; b < W / 8; ++b) {
         if (b >= nb) continue;
         if (S > 1) {
           for (int slot = 0; slot < S - 1; ++slot) {
@@ -531,7 +547,7 @@ static int w4_map3d(CUtensorMap* m, const void* base, long long K, long long row
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-template <int BN, bool DUAL, int QB>
+template <int BN, bool DUAL, int QB, int GROUPS>
 static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   constexpr int NMAT = DUAL ? 2 : 1;
   // tile height: 128, or p.th (64..128; a multiple of 8 rows for int8, of 16 for int4, so that
@@ -571,14 +587,14 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   // half of the SM's shared memory keeps every SM at one CTA of this kernel.
   size_t smem = (size_t)fixed + (size_t)stages * STAGE;
   if (smem < 120 * 1024) smem = 120 * 1024;
-  auto kern = umma_gemm_w8_kernel<BN, DUAL, QB>;
+  auto kern = umma_gemm_w8_kernel<BN, DUAL, QB, GROUPS>;
   static SmemAsk ask;
   const cudaError_t e = ask(kern, smem);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((p.F + p.th - 1) / p.th, (p.T + BN - 1) / BN, p.splitk);
-  cfg.blockDim = dim3(kW8Threads, 1, 1);
+  cfg.blockDim = dim3(w8_threads(GROUPS), 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
@@ -598,6 +614,16 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   cfg.attrs = attrs;
   cfg.numAttrs = na;
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, ta2, tb, p);
+}
+
+// Two groups of converters where a CTA has stages enough for them to take turns; one where the set-up of
+// 18 warps counts (768 x 256: 7.2 us with one group, 7.5 with two), and for int8 at 128 rows with K split,
+// where the products take as long as the conversion (4096 x 11008: 22.5 and 23.3 us).
+template <int BN, bool DUAL, int QB>
+static int w8_pick(E2hGemmParams& p, cudaStream_t stream) {
+  const int n_it = (p.K / 128 + p.splitk - 1) / p.splitk;
+  const bool two = n_it >= 8 && !(BN == 128 && QB == 8 && p.splitk > 1);
+  return two ? w8_launch<BN, DUAL, QB, 2>(p, stream) : w8_launch<BN, DUAL, QB, 1>(p, stream);
 }
 
 }  // namespace e2h
@@ -620,9 +646,9 @@ extern "C" int e2h_gemm_w8(const E2hGemmParams* pp, void* stream_v) {
     return -7;
   if (p.scale == nullptr) return -9;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  if (p.dual) return w8_launch<64, true, 8>(p, stream);
-  if (p.bn == 64) return w8_launch<64, false, 8>(p, stream);
-  return w8_launch<128, false, 8>(p, stream);
+  if (p.dual) return w8_pick<64, true, 8>(p, stream);
+  if (p.bn == 64) return w8_pick<64, false, 8>(p, stream);
+  return w8_pick<128, false, 8>(p, stream);
 }
 
 // Weight-only int4, group-wise: p.a (and p.a2) point at packed nibbles [F, K / 2] bytes (lda =
@@ -648,7 +674,7 @@ extern "C" int e2h_gemm_w4(const E2hGemmParams* pp, void* stream_v) {
     return -9;
   p.scale = nullptr;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  if (p.dual) return w8_launch<64, true, 4>(p, stream);
-  if (p.bn == 64) return w8_launch<64, false, 4>(p, stream);
-  return w8_launch<128, false, 4>(p, stream);
+  if (p.dual) return w8_pick<64, true, 4>(p, stream);
+  if (p.bn == 64) return w8_pick<64, false, 4>(p, stream);
+  return w8_pick<128, false, 4>(p, stream);
 }
