@@ -9,8 +9,8 @@
 //
 // Layouts: q [B, n_head*D] bf16, caches [max_batch, n_kv, smax, D] bf16, out [B, n_head*D] bf16.
 //
-// Work split (with more pairs than resident CTAs; with fewer, every pair is simply cut into
-// equal parts, one per CTA): the live keys of every (sequence, kv head) are cut into chunks of
+// Work split (with more pairs than resident CTAs; with fewer, every pair of more than a few chunks is
+// simply cut into equal parts, one per CTA): the live keys of every (sequence, kv head) are cut into chunks of
 // 32 keys, all chunks are numbered (sequence, head, chunk) and every CTA takes one contiguous
 // run of that numbering, the same number of chunks for all: the CTAs finish together whatever the batch,
 // the head count and the context lengths are, and a CTA pays the latency of its first loads
@@ -82,10 +82,15 @@ struct AttnWalk {
 
 // Grouped heads (four or more query heads per kv head, head size 128) run on the tensor cores: see
 // attn_chunk_mma. Partial results of a CTA: one per half-warp, or one per warp there.
+// alone: up to how many chunks of 32 keys one CTA takes a pair by itself where there are CTAs to share it.
+// Cut -> alone (us): 1 sequence x 32 heads, 2 chunks 5.7 -> 4.0, 4 chunks 6.1 -> 5.2, 5 chunks 6.2 -> 5.8, 7
+// chunks 6.4 -> 7.1; 64 query and 8 kv heads, 2 chunks 12.1 -> 5.8, 9 chunks 14.3 -> 10.7, 13 chunks 14.9 -> 19.5;
+// 4 sequences x 4 heads of 64, 2 chunks 5.7 -> 3.8.
 template <int D, int G>
 struct AttnForm {
   static constexpr bool mma = D == 128 && G >= 4 && G <= 8;
   static constexpr int slots = mma ? kWarps : kSlots;
+  static constexpr int alone = mma ? 10 : 5;
 };
 
 __device__ __forceinline__ void mma_16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -288,12 +293,13 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int total = pre[B] * n_kv;
   int per, lo, hi;
   if (fixed_parts > 0) {
-    // fewer pairs than resident CTAs: every pair is cut into fixed_parts equal parts, one per
-    // CTA (fixed_parts == 1: one CTA per pair, nothing to merge)
+    // fewer pairs than resident CTAs: every pair of more than a few chunks is cut into fixed_parts
+    // equal parts, one per CTA (fixed_parts == 1: one CTA per pair, nothing to merge)
     const int item = blockIdx.x / fixed_parts, part = blockIdx.x - item * fixed_parts;
     const int b = item / n_kv, hk = item - b * n_kv;
     const int nc = pre[b + 1] - pre[b];
-    per = (nc + fixed_parts - 1) / fixed_parts;
+    // a few chunks are not worth the partial results, the ticket and the merge (AttnForm::alone)
+    per = nc <= AttnForm<D, G>::alone ? nc : (nc + fixed_parts - 1) / fixed_parts;
     lo = pre[b] * n_kv + hk * nc + part * per;
     hi = min(pre[b] * n_kv + (hk + 1) * nc, lo + per);
   } else {
