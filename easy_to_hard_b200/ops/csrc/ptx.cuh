@@ -490,7 +490,18 @@ __device__ __forceinline__ unsigned long long e2h_globaltimer() {
 __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
+// x * sigmoid(x) of a bf16 number x, for callers that round the result to bf16: for each of the 65536
+// inputs that is the number which x / (1.f + __expf(-x)) gives (compared for all of them; against 64 bits
+// in tests/test_silu_gpu.py). The fast division has no rounding step and no slow path to branch to, so the
+// compiler interleaves the elements of a thread: 470 -> 164 ns for 8 of them, two warps a scheduler, which
+// is what the end of a gated product's tile spends its time on (batch of 64, 7B decode step: 1237 -> 1210
+// us). It returns 0 for divisors above 2^126, where the quotient still is a normal number: divisor and
+// quotient are scaled there.
+__device__ __forceinline__ float silu(float x) {
+  const float d = 1.f + __expf(-x);
+  const float s = d > 0x1p100f ? 0x1p-30f : 1.f;
+  return __fdividef(x, d * s) * s;
+}
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ float gelu_erf(float x) {
   return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
