@@ -664,8 +664,9 @@ static int umma_plan(E2hGemmParams& p) {
   // 57 -> 50 us; 2 x 22016 x 8192 gated: 169 -> 124). With fewer CTAs than SMs half a ring is too
   // little in flight, and the next launch's CTAs crowd on the SMs that have both halves free
   // (12288 x 4096 on 96 CTAs: 26 -> 32 us). What counts is CTAs with work: of 8 experts, 2 x 2752 x 2048
-  // gated, with two live ones 20.7 us at the full ring, 33.4 at half; with all eight 61 and 45. Half a
-  // ring of one stage would not overlap loads and products: it takes two beside the exchange buffer.
+  // gated, with two live ones 20.7 us at the full ring, 33.4 at half; with all eight 61 and 45 (36 with
+  // tiles of 80 rows, twice over the SMs). Half a ring of one stage would not overlap loads and
+  // products: it takes two beside the exchange buffer.
   const int xchg = xchg_bytes(p.bn, p.splitk, p.dual, p.tf);
   const int ctas = ((p.F + p.th - 1) / p.th) * p.splitk *
                    (p.n_groups > 0 ? live_groups(p) : p.n_batch > 0 ? p.n_batch : 1);

@@ -119,6 +119,30 @@ def pick_stream_tiles(F: int, K: int, bn: int, dual: bool):
     return plan and plan[0]
 
 
+def group_height(F: int, n_groups: int, group_tmax: int, T: int):
+    """Feature-tile height of a grouped product with one token tile per group, or None for 128 rows: as
+    in ``stream_plan``, the height with which the tiles of the groups cover the SMs once, or twice where
+    tiles of 128 rows are more than the SMs. Only where it is known how many groups have rows: all of
+    them, as far as T rows of group_tmax tokens tell, or the T of a single token (at most once over the
+    SMs then: the tiles of the empty groups come in between, 8 experts of 2 x 11008 x 4096 with two live
+    83 -> 93 us at twice). Guessed too low or too high the tiles fill the SMs unevenly (16 experts of
+    3456 x 2048, 6 live: 27 -> 37 us). In a chain of launches, L2 cold, us: 4 experts of 2 x 2752 x 2048
+    28.2 -> 21.0, 2 x 5504 x 2048 44.1 -> 36.3, 3456 x 2048 15.2 -> 15.0; 8 of 2 x 2752 x 2048 43.9 ->
+    35.9; two live ones of 4, one token, 2 x 5504 x 2048 28.5 -> 22.4."""
+    if group_tmax == 1:
+        groups, covers = min(n_groups, T), 1
+    elif n_groups * max(0.0, 1.0 - T / (group_tmax * n_groups)) ** group_tmax < 0.5:
+        groups, covers = n_groups, 2
+    else:
+        return None
+    tiles128 = -(-F // 128) * groups
+    if tiles128 > covers * N_SM:
+        return None
+    per_group = (N_SM if tiles128 <= N_SM else 2 * N_SM) // groups
+    th = max(64, -(-(-(-F // per_group)) // 8) * 8)
+    return th if th < 128 and -(-F // th) <= per_group else None
+
+
 ROWS_EPIS = {EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_RESIDUAL_F32, EPI_ROPE_KV}
 ROWS_GATED = {EPI_SWIGLU, EPI_DUAL_STORE}
 ROWS_MAX = 16
@@ -251,6 +275,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
         if kps <= 0:
             kps = 1 if (K % 64 or bn > 128) else 2
         tf = 128
+        if th is None and splitk == 1 and group_tmax <= bn and K % 64 == 0 and STREAM_TILES:
+            th = group_height(F, n_groups, group_tmax, T)
         # many rows per group: persistent tiles walk group after group
         persistent = n_groups <= 96 and T >= 128 * n_groups and group_tmax > 256
         if persistent:
