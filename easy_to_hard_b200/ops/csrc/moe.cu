@@ -175,50 +175,43 @@ __global__ void moe_topk_kernel(const float* z, long long ldz, int n, int E, int
     }
 }
 
-// CTA e numbers the tokens that chose expert e: place[i] for every choice i with sel[i] == e.
+// CTA e numbers the tokens that chose expert e: place[i] for every choice i with sel[i] == e. Each warp
+// walks a run of its own twice, first to count and then, knowing what the warps before it hold, to number:
+// one barrier instead of three per 1024 choices (25136 choices of 4 experts: 55 -> 5.4 us).
 __global__ void __launch_bounds__(1024)
 moe_group_kernel(const int* sel, int m, int E, int* off, int* place) {
-  __shared__ int wsum[32];
+  __shared__ int wless[32], weq[32];
   pdl_launch_dependents();
   pdl_wait_prior();
   const int e = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int run = (m + 1023) / 1024 * 32;
+  const int i0 = min(m, warp * run), i1 = min(m, i0 + run);
   int less = 0, eq = 0;
-  for (int i = threadIdx.x; i < m; i += 1024) {
+#pragma unroll 8
+  for (int i = i0 + lane; i < i1; i += 32) {
     const int s = sel[i];
     less += s < e;
     eq += s == e;
   }
-  auto sum = [&](int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) wsum[warp] = v;
-    __syncthreads();
-    int s = 0;
-    for (int k = 0; k < 32; ++k) s += wsum[k];
-    return s;
-  };
-  less = sum(less);
-  eq = sum(eq);
-  if (threadIdx.x == 0) {
-    off[e] = less;
-    if (e == E - 1) off[E] = less + eq;
+  less = __reduce_add_sync(0xffffffffu, less);
+  eq = __reduce_add_sync(0xffffffffu, eq);
+  if (lane == 0) {
+    wless[warp] = less;
+    weq[warp] = eq;
   }
-  int run = less;
-  for (int i0 = 0; i0 < m; i0 += 1024) {
-    const int i = i0 + threadIdx.x;
-    const bool hit = i < m && sel[i] == e;
+  __syncthreads();
+  less = __reduce_add_sync(0xffffffffu, wless[lane]);
+  int before = less + __reduce_add_sync(0xffffffffu, lane < warp ? weq[lane] : 0);
+  if (threadIdx.x == 1023) {
+    off[e] = less;
+    if (e == E - 1) off[E] = before + eq;
+  }
+#pragma unroll 8
+  for (int i = i0; i < i1; i += 32) {
+    const bool hit = i + lane < i1 && sel[i + lane] == e;
     const unsigned b = __ballot_sync(0xffffffffu, hit);
-    __syncthreads();
-    if (lane == 0) wsum[warp] = __popc(b);
-    __syncthreads();
-    int before = run, tot = 0;
-    for (int k = 0; k < 32; ++k) {
-      if (k < warp) before += wsum[k];
-      tot += wsum[k];
-    }
-    if (hit) place[i] = before + __popc(b & ((1u << lane) - 1));
-    run += tot;
+    if (hit) place[i + lane] = before + __popc(b & ((1u << lane) - 1));
+    before += __popc(b);
   }
 }
 
