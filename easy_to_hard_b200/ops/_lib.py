@@ -148,6 +148,7 @@ _SIGNATURES = {
     "e2h_gemm_umma": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_persistent": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_umma_plan": [C.POINTER(GemmParams), C.POINTER(C.c_int)],
+    "e2h_gemm_w8_plan": [C.POINTER(GemmParams), C.c_int, C.POINTER(C.c_int)],
     "e2h_gemm_w8": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_w4": [C.POINTER(GemmParams), _vp],
     "e2h_gemm_f32": [C.POINTER(GemmParams), _vp],

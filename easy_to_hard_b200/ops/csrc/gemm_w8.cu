@@ -46,7 +46,10 @@ constexpr int w8_threads(int groups) {   // TMA warp, MMA warp, groups of 8 conv
 constexpr int kW8MaxStages = 8;
 constexpr int kW8Ctrl = 1024;
 constexpr int kW8Kps = 2;          // 64-wide k-blocks per pipeline stage
-constexpr int kW8ConvMax = 4;      // converted-tile buffers: 4 (3 for a dual GEMM: twice as large)
+constexpr int kW8ConvMax = 4;
+constexpr int w8_buffers(bool dual) {   // converted-tile buffers (those of a dual GEMM are twice as large)
+  return dual ? 3 : kW8ConvMax;
+}
 constexpr int kW8ACol0 = 128;      // tensor-memory column of the first converted-tile buffer
 constexpr int kW8ACols = 64;       // columns of one converted [128 x 128 k] bf16 tile
 constexpr int kW8TmemCols = 512;
@@ -66,6 +69,13 @@ __host__ __device__ inline int w8_xchg_bytes(int bn, int splitk, int dual) {
   if (splitk <= 1) return 0;
   return (splitk - 1) * (bn / splitk) * 128 * 4 * (dual ? 2 : 1);
 }
+// Shared memory of one stage, and what a launch needs beside its stages.
+inline int w8_stage_bytes(const E2hGemmParams& p, int bits) {
+  return p.th * 16 * bits * (p.dual ? 2 : 1) + kW8Kps * p.bn * 128;
+}
+inline int w8_fixed_bytes(const E2hGemmParams& p) {
+  return 1024 + kW8Ctrl + w8_xchg_bytes(p.bn, p.splitk, p.dual);
+}
 
 // QB = 8: int8 weights with per-feature scales in the epilogue; QB = 4: packed int4 weights with
 // group-wise (scale, zero) pairs applied by the converters.
@@ -78,7 +88,7 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   // the conversion -> MMA -> commit round trip of one buffer takes about 2 us; several buffers
   // in flight hide it. Tensor memory: accumulators in columns [0, 128), converted tiles in
   // [128, 512): 4 buffers of 64 columns (3 of 128 for a dual GEMM).
-  constexpr int kW8Conv = DUAL ? 3 : 4;
+  constexpr int kW8Conv = w8_buffers(DUAL);
   constexpr int B_BYTES = BN * 128;
   // quantised weight tile of one stage: TH rows x 128 k. TH = p.th (64..128): with lower tiles
   // a wide layer covers (nearly) all SMs in one wave instead of leaving a third of them idle;
@@ -265,10 +275,15 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // thread (row, half): the 64 k of `row` that make up bf16 k-block `half` of the stage
     const int row = lane_row;
     const int sw = row & 7;                           // 128B-swizzle term of this row
-    const int group = (warp - 2) >> 3;                // of two, 0 takes the even stages, 1 the odd ones
+    const int group = (warp - 2) >> 3;                // of two, 0 takes the even trips, 1 the odd ones
     bool ok = true;
-    int s = stages > 1 ? group : 0;
-    uint32_t ph = stages > 1 ? 0 : group;
+    // A wait for phase k of a barrier returns at once while phase k - 1 is still under way: its parity is that of
+    // phase k - 2. Trip `it` therefore needs to know that trip it - S of its stage, S stages before, has been
+    // loaded. With S even that was the same group, which has waited for it. With S odd it was the other one; but the
+    // wait for the buffer, which comes first, says that the products of trip it - kW8Conv are done, and
+    // those of it - S with them if S >= kW8Conv. w8_groups allows two groups in these two cases only.
+    int s = group;
+    uint32_t ph = 0;
     int c = group;
     uint32_t cph = 0;
     const int gshift = QB == 4 ? __ffs(p.groupsize) - 1 : 0;   // group size is a power of two
@@ -298,17 +313,17 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int s_cur = s;
       const uint32_t ph_cur = ph;
       s += GROUPS;
-      while (s >= stages) {
+      if (s >= stages) {
         s -= stages;
         ph ^= 1;
       }
       // every converter thread waits itself (one polling lane per warp plus a shuffle measured
       // 10% slower: the acquire has to be re-established for the other lanes anyway)
       if (ok)
-        ok = mbar_wait(smem_u32(&ctrl->full[s_cur]), ph_cur, abort_flag, p.status,
-                       kStatusTimeoutFull) &&
-             mbar_wait(smem_u32(&ctrl->conv_empty[c]), cph ^ 1, abort_flag, p.status,
-                       kStatusTimeoutEmpty);
+        ok = mbar_wait(smem_u32(&ctrl->conv_empty[c]), cph ^ 1, abort_flag, p.status,
+                       kStatusTimeoutEmpty) &&
+             mbar_wait(smem_u32(&ctrl->full[s_cur]), ph_cur, abort_flag, p.status,
+                       kStatusTimeoutFull);
       tc_fence_after();
       if (ok) {
         const uint8_t* st = tiles + (size_t)s_cur * STAGE;
@@ -547,16 +562,39 @@ static int w4_map3d(CUtensorMap* m, const void* base, long long K, long long row
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-template <int BN, bool DUAL, int QB, int GROUPS>
-static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
-  constexpr int NMAT = DUAL ? 2 : 1;
+// Groups of converters of a launch with this many stages. Two where a CTA has stages enough for them to take
+// turns; one where the set-up of 18 warps counts (768 x 256: 7.2 us with one group, 7.5 with two), and for int8 at
+// 128 rows with K split, where the products take as long as the conversion (4096 x 11008: 22.5 and 23.3
+// us). Two want a ring in which no wait can take an old phase for the new one: the converters say why.
+static int w8_groups(const E2hGemmParams& p, int bits) {
+  const int n_it = (p.K / 128 + p.splitk - 1) / p.splitk;
+  if (n_it < 8 || (p.bn == 128 && bits == 8 && p.splitk > 1)) return 1;
+  return p.stages % 2 == 0 || p.stages >= w8_buffers(p.dual) ? 2 : 1;
+}
+
+// Checks the parameters and settles what a launch chooses by itself: tile height, stages and form of the
+// epilogue, in p, and the groups of converters. 0 or an error code.
+static int w8_plan(E2hGemmParams& p, int bits, int& groups) {
+  if (p.F <= 0 || p.T <= 0 || p.K <= 0 || (p.K % 128)) return -1;
+  if (p.bn != 64 && p.bn != 128) return -2;
+  if (p.dual && p.bn != 64) return -2;
+  if (p.splitk < 1 || p.splitk > 8 || (p.bn % (p.splitk * 8)) != 0) return -3;
+  if ((p.K / 128) < p.splitk) return -4;
+  if (p.a_mn_major || p.b_mn_major || p.a_tiled) return -5;
+  if (p.dual && (p.a2 == nullptr || (bits == 4 && p.qsz2 == nullptr))) return -5;
+  if ((p.lda % 16) || (p.ldb % 8) || (p.dual && (p.lda2 % 16))) return -6;
+  if (((uintptr_t)p.a & 15) || ((uintptr_t)p.b & 15) || (p.dual && ((uintptr_t)p.a2 & 15)))
+    return -7;
+  if (bits == 8 ? p.scale == nullptr
+                : p.qsz == nullptr || p.groupsize < 64 || (p.groupsize & (p.groupsize - 1)) ||
+                      (p.K % p.groupsize))
+    return -9;
   // tile height: 128, or p.th (64..128; a multiple of 8 rows for int8, of 16 for int4, so that
   // every part of a stage starts on a swizzle-atom boundary)
   if (p.th <= 0) p.th = 128;
-  if (p.th < 64 || p.th > 128 || (p.th % (QB == 8 ? 8 : 16))) return -12;
-  const int STAGE = p.th * 16 * QB * NMAT + kW8Kps * BN * 128;
-  const int fixed = 1024 + kW8Ctrl + w8_xchg_bytes(BN, p.splitk, DUAL);
-  int stages = (227 * 1024 - fixed) / STAGE;
+  if (p.th < 64 || p.th > 128 || (p.th % (bits == 8 ? 8 : 16))) return -12;
+  const int stage = w8_stage_bytes(p, bits);
+  int stages = (227 * 1024 - w8_fixed_bytes(p)) / stage;
   if (stages > kW8MaxStages) stages = kW8MaxStages;
   if (p.stages > 0 && p.stages < stages) stages = p.stages;
   const int n_it = (p.K / 128 + p.splitk - 1) / p.splitk;
@@ -566,8 +604,14 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   // staged (shared-memory) epilogue when the output layout allows 16-byte accesses and the
   // finished tile fits the pipeline buffers it reuses
   p.stage_epi = (epi_can_stage(p, p.th) &&
-                 (long long)(BN / p.splitk) * p.th * 2 <= (long long)stages * STAGE)
+                 (long long)(p.bn / p.splitk) * p.th * 2 <= (long long)stages * stage)
                     ? 1 : 0;
+  groups = w8_groups(p, bits);
+  return 0;
+}
+
+template <int BN, bool DUAL, int QB, int GROUPS>
+static int w8_launch(const E2hGemmParams& p, cudaStream_t stream) {
   CUtensorMap ta, ta2, tb;
   int r = QB == 8 ? w8_map3d(&ta, p.a, p.K, p.F, p.lda, p.th, 1, true)
                   : w4_map3d(&ta, p.a, p.K, p.F, p.lda, p.th);
@@ -585,7 +629,7 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   // running CTA, not by the launch: a second CTA of the same cluster on the same SM would wait
   // for columns that its partner only frees after the cluster barrier. Asking for more than
   // half of the SM's shared memory keeps every SM at one CTA of this kernel.
-  size_t smem = (size_t)fixed + (size_t)stages * STAGE;
+  size_t smem = (size_t)w8_fixed_bytes(p) + (size_t)p.stages * w8_stage_bytes(p, QB);
   if (smem < 120 * 1024) smem = 120 * 1024;
   auto kern = umma_gemm_w8_kernel<BN, DUAL, QB, GROUPS>;
   static SmemAsk ask;
@@ -616,39 +660,46 @@ static int w8_launch(E2hGemmParams& p, cudaStream_t stream) {
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, ta2, tb, p);
 }
 
-// Two groups of converters where a CTA has stages enough for them to take turns; one where the set-up of
-// 18 warps counts (768 x 256: 7.2 us with one group, 7.5 with two), and for int8 at 128 rows with K split,
-// where the products take as long as the conversion (4096 x 11008: 22.5 and 23.3 us).
-template <int BN, bool DUAL, int QB>
-static int w8_pick(E2hGemmParams& p, cudaStream_t stream) {
-  const int n_it = (p.K / 128 + p.splitk - 1) / p.splitk;
-  const bool two = n_it >= 8 && !(BN == 128 && QB == 8 && p.splitk > 1);
-  return two ? w8_launch<BN, DUAL, QB, 2>(p, stream) : w8_launch<BN, DUAL, QB, 1>(p, stream);
+template <int BN, bool DUAL>
+static int w8_dispatch(const E2hGemmParams& p, int bits, int groups, cudaStream_t stream) {
+  if (bits == 8)
+    return groups == 2 ? w8_launch<BN, DUAL, 8, 2>(p, stream) : w8_launch<BN, DUAL, 8, 1>(p, stream);
+  return groups == 2 ? w8_launch<BN, DUAL, 4, 2>(p, stream) : w8_launch<BN, DUAL, 4, 1>(p, stream);
+}
+
+static int w8_gemm(E2hGemmParams& p, int bits, cudaStream_t stream) {
+  int groups = 1;
+  const int bad = w8_plan(p, bits, groups);
+  if (bad) return bad;
+  if (p.dual) return w8_dispatch<64, true>(p, bits, groups, stream);
+  if (p.bn == 64) return w8_dispatch<64, false>(p, bits, groups, stream);
+  return w8_dispatch<128, false>(p, bits, groups, stream);
 }
 
 }  // namespace e2h
+
+// What e2h_gemm_w8 (bits 8) or e2h_gemm_w4 (bits 4) would launch, without a GPU: out = {tile height, stages,
+// groups of converters, converted-tile buffers, staged epilogue}.
+extern "C" int e2h_gemm_w8_plan(const E2hGemmParams* pp, int bits, int* out) {
+  using namespace e2h;
+  E2hGemmParams p = *pp;
+  int groups = 1;
+  const int bad = w8_plan(p, bits, groups);
+  if (bad) return bad;
+  out[0] = p.th;
+  out[1] = p.stages;
+  out[2] = groups;
+  out[3] = w8_buffers(p.dual);
+  out[4] = p.stage_epi;
+  return 0;
+}
 
 // Same parameter block as e2h_gemm_umma, with p.a (and p.a2) pointing at int8 [F, K] weights
 // (lda in elements = bytes, a multiple of 16), p.b bf16 [T, K], K % 128 == 0, T-tile bn 64 or 128,
 // and p.scale the fp32 per-feature scales (F of them, or 2F for a dual GEMM).
 extern "C" int e2h_gemm_w8(const E2hGemmParams* pp, void* stream_v) {
-  using namespace e2h;
   E2hGemmParams p = *pp;
-  if (p.F <= 0 || p.T <= 0 || p.K <= 0 || (p.K % 128)) return -1;
-  if (p.bn != 64 && p.bn != 128) return -2;
-  if (p.dual && p.bn != 64) return -2;
-  if (p.splitk < 1 || p.splitk > 8 || (p.bn % (p.splitk * 8)) != 0) return -3;
-  if ((p.K / 128) < p.splitk) return -4;
-  if (p.a_mn_major || p.b_mn_major || p.a_tiled) return -5;
-  if (p.dual && p.a2 == nullptr) return -5;
-  if ((p.lda % 16) || (p.ldb % 8) || (p.dual && (p.lda2 % 16))) return -6;
-  if (((uintptr_t)p.a & 15) || ((uintptr_t)p.b & 15) || (p.dual && ((uintptr_t)p.a2 & 15)))
-    return -7;
-  if (p.scale == nullptr) return -9;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  if (p.dual) return w8_pick<64, true, 8>(p, stream);
-  if (p.bn == 64) return w8_pick<64, false, 8>(p, stream);
-  return w8_pick<128, false, 8>(p, stream);
+  return e2h::w8_gemm(p, 8, static_cast<cudaStream_t>(stream_v));
 }
 
 // Weight-only int4, group-wise: p.a (and p.a2) point at packed nibbles [F, K / 2] bytes (lda =
@@ -657,24 +708,7 @@ extern "C" int e2h_gemm_w8(const E2hGemmParams* pp, void* stream_v) {
 // (scale, zero) pairs of the reference's checkpoint format; p.groupsize a power of two >= 64
 // that divides K; K % 128 == 0. out = epilogue( sum_k x[t,k] * bf16((q-8) * scale + zero) ).
 extern "C" int e2h_gemm_w4(const E2hGemmParams* pp, void* stream_v) {
-  using namespace e2h;
   E2hGemmParams p = *pp;
-  if (p.F <= 0 || p.T <= 0 || p.K <= 0 || (p.K % 128)) return -1;
-  if (p.bn != 64 && p.bn != 128) return -2;
-  if (p.dual && p.bn != 64) return -2;
-  if (p.splitk < 1 || p.splitk > 8 || (p.bn % (p.splitk * 8)) != 0) return -3;
-  if ((p.K / 128) < p.splitk) return -4;
-  if (p.a_mn_major || p.b_mn_major || p.a_tiled) return -5;
-  if (p.dual && (p.a2 == nullptr || p.qsz2 == nullptr)) return -5;
-  if ((p.lda % 16) || (p.ldb % 8) || (p.dual && (p.lda2 % 16))) return -6;
-  if (((uintptr_t)p.a & 15) || ((uintptr_t)p.b & 15) || (p.dual && ((uintptr_t)p.a2 & 15)))
-    return -7;
-  if (p.qsz == nullptr || p.groupsize < 64 || (p.groupsize & (p.groupsize - 1)) ||
-      (p.K % p.groupsize))
-    return -9;
   p.scale = nullptr;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  if (p.dual) return w8_pick<64, true, 4>(p, stream);
-  if (p.bn == 64) return w8_pick<64, false, 4>(p, stream);
-  return w8_pick<128, false, 4>(p, stream);
+  return e2h::w8_gemm(p, 4, static_cast<cudaStream_t>(stream_v));
 }

@@ -143,6 +143,19 @@ def group_height(F: int, n_groups: int, group_tmax: int, T: int):
     return th if th < 128 and -(-F // th) <= per_group else None
 
 
+def quant_height(F: int, bits: int) -> int:
+    """Feature-tile height of an int8 / int4 product whose K is not split, or 0 for 128 rows: the
+    converting kernel is bound by bytes in flight per SM, so one that puts a CTA on (nearly) every
+    SM; rows per tile a multiple of 8 (int8) or 16 (int4)."""
+    q = 16 if bits == 4 else 8
+    tiles128 = -(-F // 128)
+    if tiles128 * 2 > N_SM and tiles128 <= N_SM:
+        cand = max(64, min(128, -(-(-(-F // N_SM)) // q) * q))
+        if -(-F // cand) <= N_SM:
+            return cand
+    return 0
+
+
 ROWS_EPIS = {EPI_STORE_BF16, EPI_STORE_F32, EPI_RESIDUAL, EPI_RESIDUAL_F32, EPI_ROPE_KV}
 ROWS_GATED = {EPI_SWIGLU, EPI_DUAL_STORE}
 ROWS_MAX = 16
@@ -306,14 +319,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, epi: int, out: Optional[torch.Tens
             stage = _smem_bytes(bn, th, dual, splitk, 2, 4)
             kps = 4 if stage <= 227 * 1024 else 2
     if (w8 or w4) and not th and splitk == 1 and STREAM_TILES:
-        # the converting kernel is bound by bytes in flight per SM: a tile height that puts a
-        # CTA on (nearly) every SM; rows per tile a multiple of 8 (int8) or 16 (int4)
-        q = 16 if w4 else 8
-        tiles128 = -(-F // 128)
-        if tiles128 * 2 > N_SM and tiles128 <= N_SM:
-            cand = max(64, min(128, -(-(-(-F // N_SM)) // q) * q))
-            if -(-F // cand) <= N_SM:
-                th = cand
+        th = quant_height(F, 4 if w4 else 8)
     p = GemmParams()
     p.F, p.T, p.K = F, T, K
     p.splitk, p.epi, p.stages = splitk, epi, stages

@@ -73,3 +73,31 @@ def test_every_code():
         x[torch.arange(64), first + torch.arange(64)] = 1
         gemm.linear(x, w, out=out, scale=torch.ones(256, device="cuda"))
         assert torch.equal(out, w[0, first:first + 64].float()[:, None].expand(64, 256))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("dual,T", [(False, 40), (False, 100), (True, 64)])
+@pytest.mark.parametrize("ring", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("trips", [8, 19])
+def test_rings(bits, dual, T, ring, trips):
+    """Rings of so many stages (all of them fit): odd ones, and ones with fewer stages than converted-tile
+    buffers. A stage converted before its load has landed gives what an earlier trip held."""
+    from easy_to_hard_b200.ops import _lib, gemm
+    F, K = 9600, 128 * trips
+    g = torch.Generator(device="cuda").manual_seed(K + T)
+    ws = [_weight(F, K, bits, g) for _ in range(1 + dual)]
+    x = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    scale = torch.cat([s for _, s, _ in ws]) if bits == 8 else None
+    wf = [f if s is None else f * s.double()[:, None] for _, s, f in ws]
+    outs = [torch.empty(T, F, device="cuda", dtype=torch.bfloat16 if dual else torch.float32) for _ in ws]
+    for _ in range(4):
+        if dual:
+            gemm.gemm(ws[0][0], x, epi=gemm.EPI_DUAL_STORE, a2=ws[1][0], out=outs[0], out2=outs[1], scale=scale,
+                      stages=ring)
+        else:
+            gemm.gemm(ws[0][0], x, epi=gemm.EPI_STORE_F32, out=outs[0], scale=scale, stages=ring)
+        for out, f in zip(outs, wf):
+            want = x.double() @ f.t()
+            tol = (K + 2) * 2.0 ** -23 * (x.double().abs() @ f.abs().t()) + 2.0 ** -8 * dual * want.abs()
+            assert bool(((out.double() - want).abs() <= 1.01 * tol + 1e-30).all())
+    assert _lib.read_status() == 0
