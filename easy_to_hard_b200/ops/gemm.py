@@ -129,6 +129,8 @@ def group_height(F: int, n_groups: int, group_tmax: int, T: int):
     3456 x 2048, 6 live: 27 -> 37 us). In a chain of launches, L2 cold, us: 4 experts of 2 x 2752 x 2048
     28.2 -> 21.0, 2 x 5504 x 2048 44.1 -> 36.3, 3456 x 2048 15.2 -> 15.0; 8 of 2 x 2752 x 2048 43.9 ->
     35.9; two live ones of 4, one token, 2 x 5504 x 2048 28.5 -> 22.4."""
+    if T <= 0 or group_tmax <= 0:
+        return None                       # (nothing to cover: the launch refuses it)
     if group_tmax == 1:
         groups, covers = min(n_groups, T), 1
     elif n_groups * max(0.0, 1.0 - T / (group_tmax * n_groups)) ** group_tmax < 0.5:

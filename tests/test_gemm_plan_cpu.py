@@ -147,3 +147,17 @@ def test_int4_pairs_of_another_layout_go_through_the_general_expansion(launches,
             gemm.linear(x, w, out=out)
             assert len(launches) == 1 and len(expanded) == 1
         assert not gemm.rows_rule(w, None, x, gemm.EPI_STORE_BF16)
+
+
+@pytest.mark.parametrize("T,tmax", [(0, 0), (0, 1), (0, 8), (4, 0)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_grouped_products_without_rows_are_refused_by_the_launch(launches, T, tmax, gated):
+    K, F, n = 256, 904, 4
+    x, out = (OnGpu(torch.zeros(T, width, dtype=torch.bfloat16)) for width in (K, F))
+    w = OnGpu(torch.zeros(n * F, K, dtype=torch.bfloat16))
+    off = torch.zeros(n + 1, dtype=torch.int32)
+    if gated:
+        gemm.grouped_swiglu(x, w, w, out, off, n, tmax)
+    else:
+        gemm.grouped_linear(x, w, out, off, n, tmax)
+    assert len(launches) == 1 and _plan(launches[0]) < 0
