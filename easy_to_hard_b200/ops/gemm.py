@@ -122,13 +122,25 @@ def pick_stream_tiles(F: int, K: int, bn: int, dual: bool):
 def group_height(F: int, n_groups: int, group_tmax: int, T: int):
     """Feature-tile height of a grouped product with one token tile per group, or None for 128 rows: as
     in ``stream_plan``, the height with which the tiles of the groups cover the SMs once, or twice where
-    tiles of 128 rows are more than the SMs. Only where it is known how many groups have rows: all of
+    tiles of 128 rows are more than the SMs. Only where it can be told how many groups have rows: all of
     them, as far as T rows of group_tmax tokens tell, or the T of a single token (at most once over the
     SMs then: the tiles of the empty groups come in between, 8 experts of 2 x 11008 x 4096 with two live
-    83 -> 93 us at twice). Guessed too low or too high the tiles fill the SMs unevenly (16 experts of
-    3456 x 2048, 6 live: 27 -> 37 us). In a chain of launches, L2 cold, us: 4 experts of 2 x 2752 x 2048
-    28.2 -> 21.0, 2 x 5504 x 2048 44.1 -> 36.3, 3456 x 2048 15.2 -> 15.0; 8 of 2 x 2752 x 2048 43.9 ->
-    35.9; two live ones of 4, one token, 2 x 5504 x 2048 28.5 -> 22.4."""
+    83 -> 93 us at twice). 16 experts of 3456 x 2048 with six live are no such case (27 -> 37 us).
+    Measured in a chain of launches, L2 cold, tiles of 128 rows -> lower ones, us, experts of K 2048:
+
+        experts, features, tokens      64-token tile    128          256
+        4 of 2752 (80 rows)            13.9 -> 13.4     16.7 -> 15.5  26.6 -> 24.8
+        4 of 2 x 2752, gated (80)      24.5 -> 21.7     28.3 -> 25.1
+        8 of 2752 (80)                 22.1 -> 21.2     25.4 -> 23.9  51.1 -> 48.6
+        8 of 2 x 2752, gated (80)      41.2 -> 37.1     46.5 -> 41.7
+        4 of 3456 (96)                 15.0 -> 14.7     17.8 -> 16.6  27.0 -> 25.4
+        4 of 2 x 3456, gated (96)      26.9 -> 25.0     30.4 -> 30.0
+
+    Heights of 104 and 112 are at 0.92 to 1.02 of the time with 128 rows (8 experts of 1768 to 2016 features,
+    K of 1024 and 4096), 120 gained nowhere and lost up to 4 % (2048 x 1024 12.1 -> 12.5). Tokens that
+    leave experts empty change little: of 8 gated experts of 2 x 2752 with 2, 4 and 6 live 31.6 -> 23.9, 34.2 ->
+    25.6, 37.2 -> 31.3, ungated 18.8 -> 18.4, 18.9 -> 18.8, 19.4 -> 19.9; popularities of 1 / rank^1.5 as
+    above."""
     if T <= 0 or group_tmax <= 0:
         return None                       # (nothing to cover: the launch refuses it)
     if group_tmax == 1:
@@ -142,7 +154,7 @@ def group_height(F: int, n_groups: int, group_tmax: int, T: int):
         return None
     per_group = (N_SM if tiles128 <= N_SM else 2 * N_SM) // groups
     th = max(64, -(-(-(-F // per_group)) // 8) * 8)
-    return th if th < 128 and -(-F // th) <= per_group else None
+    return th if th <= 112 and -(-F // th) <= per_group else None
 
 
 def quant_height(F: int, bits: int) -> int:

@@ -64,3 +64,29 @@ def test_low_tiles(F, K, n, tokens, top, gated):
             tol = tol + U * (want.abs() + tol)
         assert ((out[a:b].double() - want).abs() <= 1.001 * tol + 1e-30).all()
     assert (out[int(off[-1]):] == 7.0).all()                   # rows of no group stay as they were
+
+
+# token tiles of 128 and of 256 rows, at their edges
+WIDE = [(2752, 256, 4, 65, 2), (904, 192, 8, 100, 2), (1776, 128, 8, 128, 2), (1368, 320, 4, 129, 3),
+        (2752, 128, 4, 200, 2), (1104, 128, 5, 256, 2)]
+
+
+@pytest.mark.parametrize("F,K,n,tokens,top", WIDE)
+def test_heights_are_low_for_wide_token_tiles(F, K, n, tokens, top):
+    test_heights_are_low(F, K, n, tokens, top)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("F,K,n,tokens,top", WIDE)
+def test_low_tiles_of_many_tokens(F, K, n, tokens, top, gated):
+    test_low_tiles(F, K, n, tokens, top, gated)
+
+
+def test_heights_that_gain_nothing_are_left_out():
+    """Groups whose tiles of 128 rows cover the SMs nearly as well keep them."""
+    for F in range(64, 6000, 8):
+        for n in (1, 4, 5, 8, 16):
+            th = gemm.group_height(F, n, 32, 32 * n)
+            assert th is None or 64 <= th <= 112
+    assert gemm.group_height(2048, 8, 16, 32) is None
