@@ -92,7 +92,6 @@ class ShardUnit:
         del flat
         for p in self.params:             # the full tensors only exist while gathered
             p.data = torch.empty(0, dtype=compute_dtype, device=dev)
-        self.gathered_in: Optional[torch.Tensor] = None
         self.lp_symm = None        # (SymmetricBuffer, byte offset) once shard_lp lives in one
         self.lp_peers = None       # index of each rank of this group inside that buffer's group
 
@@ -109,12 +108,12 @@ class ShardUnit:
         self.lp_symm = (sbuf, offset)
 
     # -------------------------------------------------------------- parameters
-    def gather_into(self, buf: torch.Tensor) -> None:
+    def gather_into(self, buf: Optional[torch.Tensor]) -> None:
         """All-gather the bf16 shards into ``buf`` and point the parameters at views of it. A single
-        rank's shard is the whole: the parameters are views of the shard itself, which only an optimizer
-        step writes, in the order of the stream that the blocks run on (the copies took 0.5 ms of an
-        11 ms step of one 13B layer)."""
-        full = buf[: self.padded]
+        rank's shard is the whole: it needs no ``buf``, and the parameters are views of the shard itself.
+        That is written by an optimizer step and by loading a state only, in the order of the stream
+        that the blocks run on (the copies took 0.5 ms of an 11 ms step of one 13B layer)."""
+        full = self.shard_lp if self.world == 1 else buf[: self.padded]
         if self.world > 1 and self.lp_symm is not None:
             # pull every rank's bf16 shard straight out of its symmetric memory (NVLink loads in
             # our own kernel); the shards only change at optimizer steps, which are fenced by
@@ -132,16 +131,12 @@ class ShardUnit:
             _lib.check(rc, "p2p_all_gather")
         elif self.world > 1:
             dist.all_gather_into_tensor(full, self.shard_lp, group=self.group)
-        else:
-            full = self.shard_lp
         for p, o, n, shp in zip(self.params, self.offsets, self.numels, self.shapes):
             p.data = full[o:o + n].view(shp)
-        self.gathered_in = buf
 
     def release(self) -> None:
         for p in self.params:
             p.data = torch.empty(0, dtype=self.compute_dtype, device=p.device)
-        self.gathered_in = None
 
     def grad_views(self, gradbuf: torch.Tensor) -> Dict[str, torch.Tensor]:
         full = gradbuf[: self.padded]
@@ -293,7 +288,9 @@ class ShardedDataParallel(nn.Module):
                                   reduce_dtype if self.fused else param_dtype)
         self._shards = nn.ParameterList([u.shard for u in self._all_units()])
         biggest = max(u.padded for u in self._all_units())
-        if keep_params:      # one resident buffer per block
+        if self.world == 1:  # the parameters are views of the shards
+            self._param_bufs = []
+        elif keep_params:    # one resident buffer per block
             self._param_bufs = [torch.empty(u.padded, dtype=self.compute_dtype, device=dev)
                                 for u in self.units]
         else:                # two rotating buffers: the block in use and the prefetched one
@@ -322,8 +319,8 @@ class ShardedDataParallel(nn.Module):
                 self._lp_bar = P2PChannel(256, process_group)
                 self._lp_bar.barrier()      # every rank's shards are in place
         self._root_buf = (torch.empty(self.root.padded, dtype=self.compute_dtype, device=dev)
-                          if self.root else None)
-        self._comm_stream = torch.cuda.Stream() if dev.type == "cuda" else None
+                          if self.root and self.world > 1 else None)
+        self._comm_stream = torch.cuda.Stream() if dev.type == "cuda" and self.world > 1 else None
         # the gradient reduce-scatter of block i runs on its own stream, under the backward
         # GEMMs of block i-1 (E2H_RS_OVERLAP=0 keeps it on the compute stream)
         import os
@@ -388,7 +385,7 @@ class ShardedDataParallel(nn.Module):
             self._pending[idx] = None       # still gathered from an earlier use of this step
             return
         unit = self.units[idx]
-        buf = self._param_bufs[idx if self.keep_params else idx % 2]
+        buf = self._param_bufs[idx if self.keep_params else idx % 2] if self._param_bufs else None
         self._resident[idx] = self.keep_params
         self.gathers += 1
         if self._comm_stream is None:
