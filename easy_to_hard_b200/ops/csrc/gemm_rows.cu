@@ -338,6 +338,8 @@ static int rows_dispatch(const E2hGemmParams& p, int mt, int ctas, int warps, bo
   }
   if constexpr (QB == 8 || (QB == 16 && NT == 1)) {
     if (share && mt == 2) return rows_launch<QB, 2, NT, false, 12288, true>(p, ctas, warps, stream);
+  }
+  if constexpr (QB != 4 && NT == 1) {
     if (share) return rows_launch<QB, 1, NT, false, 12288, true>(p, ctas, warps, stream);
   }
   if (mt == 2) return rows_launch<QB, 2, NT, false, 12288, false>(p, ctas, warps, stream);
@@ -385,21 +387,31 @@ extern "C" int e2h_gemm_rows(const E2hGemmParams* pp, int bits, void* stream_v) 
   const int mt = p.F >= 32 * 148 * (wide ? 1 : 2) ? 2 : 1;     // (rows_pays in ops/gemm.py knows this)
   const int ft = p.dual ? 16 : 16 * mt;
   const int tiles = (p.F + ft - 1) / ft;
-  // Three to six tiles a SM: as many CTAs there, with equal shares of the features. With whole tiles some SMs
+  // Three or four tiles a SM: as many CTAs there, with equal shares of the features. With whole tiles some SMs
   // had one more than others, and with more CTAs than fit at once a last round ran half empty (12288
   // features are 384 tiles on 296 places). bf16, up to 8 rows: three a SM fit at once with a ring of 8 KB, four
-  // make two rounds with 12 KB. Not for int4, whose time goes with the tiles' arithmetic, used rows or
-  // not (5120 x 13824, 8 rows 25.7 -> 38.8 us), nor for gated products; with one or two tiles, or seven and
-  // more, shares lost 3 to 5 %, as for bf16 from 9 rows on and for long sums in int8. us at 1 and 8 rows: 12288 x 4096 bf16 20.9 -> 17.3 and 22.1 -> 17.9, int8 14.7
-  // -> 13.2 and 15.3 -> 13.8 (16 rows 19.7 -> 15.8); 5120 x 5120 bf16 13.6 -> 10.7 and 14.6 -> 11.8, int8 11.1
-  // -> 10.1; 5760 x 2048 bf16 8.8 -> 6.7 and 9.8 -> 7.5.
+  // make two rounds with 12 KB. us with whole tiles -> shares, one row (eight rows gain alike):
+  //     bf16 5120 x 5120 (3 of 16) 13.9 -> 11.7   12288 x 4096 (3 of 32) 21.6 -> 18.1   13824 x 16384 66.6 -> 69.8
+  //          8192 x 4096 (4 of 16) 14.9 -> 13.3   15360 x 5120 (4 of 32) 28.3 -> 26.9   8192 x 11008 32.0 -> 30.4
+  //     int8 12288 x 4096 0.90 of the time, 5120 x 4096 0.93, 15360 x 4096 0.88, 16 rows 12288 x 4096 0.85
+  // Eight warps for four tiles a SM from where their longer sums pay: tiles of 32 features from K = 4096 on
+  // (15360 x 4096 four warps 1.02, eight 0.97 of the time with whole tiles; x 2048 0.89 and 1.00), tiles of 16
+  // from 12288 on (9216 x 8192 0.95 and 1.04, x 16384 1.08 and 1.02). Where shares gain nothing:
+  //   - five and six tiles a SM: bf16 0.97 to 1.07, int8 0.96 to 1.08; one or two, and seven and more, lost 3 to 5 %
+  //   - int8 tiles of 16 with K above 8192 (5120 x 8192 0.97, x 11008 1.02, x 16384 1.04); tiles of 32 gain up
+  //     to 16384 (0.95 to 0.99)
+  //   - int8 from 9 rows on, but for three tiles of 32 (0.82 to 0.85 from K = 4096 on; four 1.00 to 1.04); bf16 there
+  //   - int4, whose time goes with the tiles' arithmetic, used rows or not (5120 x 13824, 8 rows 25.7 -> 38.8 us),
+  //     and gated products
   const int per_sm = (tiles + 147) / 148;
-  const bool share = !p.dual && per_sm >= 3 && per_sm <= 6 &&
-                     (bits == 16 ? p.T <= 8 : bits == 8 && p.K <= 8192);
+  const bool share = !p.dual && (per_sm == 3 || per_sm == 4) &&
+                     (bits == 16  ? p.T <= 8
+                      : bits == 8 ? (p.T <= 8 ? mt == 2 || p.K <= 8192 : mt == 2 && per_sm == 3)
+                                  : false);
   const int ctas = share ? 148 * per_sm : tiles;
   const bool short_ring = share && bits == 16 && per_sm == 3;
   int warps = tiles >= 148 * (p.T > 8 || share ? 2 : 4) ? 4 : 8;
-  if (short_ring || (share && bits == 16 && per_sm == 4 && p.K >= 4096)) warps = 8;
+  if (short_ring || (share && bits == 16 && p.K >= (mt == 2 ? 4096 : 12288))) warps = 8;
   while (warps > 2 && units < 2 * warps) warps >>= 1;    // (the epilogue of 16 rows takes two)
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 #define E2H_ROWS(QB_)                                                                           \

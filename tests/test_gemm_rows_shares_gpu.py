@@ -57,3 +57,12 @@ def test_rotation(H, G, D):
     assert bool(((got - turned).abs() <= 2.0 ** -8 * (mag + turned.abs()) + 1e-3).all())
     assert bool(((vc[:, :, pos].flatten(1).double() - y[:, (H + G) * D:]).abs()
                  <= 2.0 ** -8 * y[:, (H + G) * D:].abs() + 1e-3).all())
+
+
+@pytest.mark.parametrize("T", [1, 16])
+@pytest.mark.parametrize("bits", [16, 8])
+@pytest.mark.parametrize("F", [16 * SM * 3, 16 * SM * 4 - 1, 32 * SM * 3, 32 * SM * 4 - 2])
+@pytest.mark.parametrize("K", [2048, 8192, 8208, 12288])
+def test_shares_of_long_sums(T, bits, F, K):
+    """On both sides of the lengths at which a product leaves the shares or takes eight warps."""
+    test_shares(T, bits, F, K)
