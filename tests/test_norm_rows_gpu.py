@@ -59,3 +59,28 @@ def test_embedding_rows(T, d):
     for t in (T // 2, T - 1):
         assert not h[t].any() and not x[t].any()
     assert _lib.read_status() == 106
+
+
+@pytest.mark.parametrize("T", [1, 255, 257, 2369, 5015])
+@pytest.mark.parametrize("d", [256, 1032, 4096, 8192])
+def test_in_place(T, d):
+    """The result over one of its inputs: each block loads its next row before it stores this one, and no
+    row is another block's."""
+    from easy_to_hard_b200.ops import _lib, functional as Fn
+    x, dy, res, w = _data(T, d, 3)
+    p = lambda t: t.data_ptr()
+
+    def bwd(a, b, r, out):
+        _lib.check(_lib.lib().e2h_rmsnorm_bwd(p(a), p(b), p(w), p(r), p(out), T, d, 1e-5, _lib.stream()), "bwd")
+        return out
+    want = bwd(x, dy, res, torch.empty_like(x))
+    for k in range(3):
+        args = [x.clone(), dy.clone(), res.clone()]
+        assert torch.equal(bwd(*args, args[k]), want)
+    want = Fn.rmsnorm(x, w, 1e-5)
+    y = x.clone()
+    _lib.check(_lib.lib().e2h_rmsnorm_fwd(p(y), None, None, 0, None, 0, p(w), None, p(y), None, T, d, 1e-5,
+                                          None, None, None, _lib.status_word(x.device).data_ptr(),
+                                          _lib.stream()), "fwd")
+    assert torch.equal(y, want)
+    assert _lib.read_status() == 0
