@@ -61,14 +61,21 @@ constexpr float kRescaleThreshold = 8.f;   // log2 units: P stays below 2^8 betw
 // stale maximum keeps being used, which is exact after the final division by the row sum. Score tiles
 // that lie entirely below the diagonal and right of the left-pad boundary skip the visibility tests.
 //
-// What bounds it: 16 exponentials per cycle and SM (512 cycles per 128 x 64 scores) beside products that take
-// 640 (Q K^T at N = 64 is bound by its operands' 6 KB of shared memory); measured about 1600 per pair of
-// such tiles, the rest being hand-overs between the roles. Time per launch, one 128-query tile per CTA
-// with two threads per row and P through shared memory -> this:
-//   64 sequences x 768, 32 heads             849 -> 482 us       16 x 768, 32 heads              225 -> 133
+// What bounds it: a pair step, 64 keys of both query tiles, has 1280 cycles of products (of each tile Q K^T at
+// N = 64 takes 384, bound by its operands' 6 KB of shared memory, and P V 256) beside 1024 of exponentials
+// (16 per cycle and SM). Measured about 1950 a step in long rows (1 x 16000: 0.56 of the burst rate), the rest being
+// hand-overs between the roles. Beside its steps an item costs 6000 to 7000: its queries, first scores, last
+// products and outputs wait for one another, and only the other query tile fills in. At 768 tokens, 8 steps
+// an item, that makes 2750 a step (profiles/flash_fwd_b4_s768_h32_d128.md; 0.37 to 0.39 of the burst rate).
+// us per launch, one 128-query tile per CTA with two threads per row and P through shared memory -> this:
+//   64 sequences x 768, 32 heads             849 -> 482          16 x 768, 32 heads              225 -> 133
 //   32 x 701, 64 query and 8 kv heads        834 -> 423          5 x 1003, 40 heads              142 -> 91
 //   4 x 4000, 32 heads, left pads            547 -> 370          1 x 4000, 32 heads              206 -> 166
 //   2 x 8000, 32 heads                      1232 -> 1074         64 x 61, 32 heads                93 -> 60
+// Launch after launch it runs into the power cap (1.5 to 1.9 GHz, the older form 1.7 to 1.97), and the gain is
+// smaller: 64 x 768 858 -> 508, 16 x 768 225 -> 161, 1 x 4000 216 -> 207, 2 x 8000 1390 -> 1260. Head size 64, the
+// same way: 64 x 768 749 -> 446, 16 x 768 193 -> 116, 32 x 701 726 -> 378, 4 x 4000 602 -> 387, 2 x 8000 1192 -> 888,
+// 64 x 61 78 -> 46.
 // Tried: key tiles of 128 with one buffer of scores (the tile's softmax and products wait for each other: 64 x
 // 768 646 us with a thread per row, 567 with two), a vote after each barrier wait of the issuers (546).
 __device__ __forceinline__ float max3(float a, float b, float c) {

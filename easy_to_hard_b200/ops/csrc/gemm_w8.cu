@@ -427,7 +427,10 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // columns of this warp: with 64 or more, alternate groups of W; with fewer, the first /
     // second half of the 8-column units
     const int units = slice >> 3;
-    constexpr int W = DUAL ? 16 : 32;    // columns per trip (two accumulators of 32 would not fit the registers)
+    // columns per trip. 18 warps leave a thread 96 registers: with two accumulators of 32 columns the gated
+    // kernels would spill in earnest. The others spill 84 to 108 bytes, outside the k-loop: 16 columns take
+    // that to 8 and no time away (12288 x 4096 int8, 64 rows 22.2 and 22.1 us, 128 rows 25.7 and 25.7).
+    constexpr int W = DUAL ? 16 : 32;
     int c_first, c_last;
     if (units >= 8) {
       c_first = W * half;

@@ -180,10 +180,14 @@ def rows_pays(F: int, K: int, T: int, bits: int) -> bool:
     tcgen05 ones. A tile of 16 or 32 features reads all rows there, where 128 features share them here:
     the more K T, the less the saved set-up of 5 us counts, and a last round of tiles that leaves SMs
     idle costs more. With tiles of 32 features and eight warps (csrc/gemm_rows.cu) the reads are no
-    bound. 16 rows, us there / here: bf16 4096 x 4096 10.3 / 12.4, 4096 x 11008 22.8 / 22.0, 8192 x 22016
-    63.4 / 64.6, 5120 x 13824 (160 tiles on 148 SMs) 36.1 / 29.6; int4 4096 x 8192 18.1 / 17.4, 8192 x
-    22016 53.6 / 64.9, 1536 x 4096 (96 tiles) 9.4 / 8.8. Over 1300 products of 512 to 32000 features
-    and K of 512 to 22016 the rule is within 0.3 % of the better choice on average, 14 % at most."""
+    bound. 16 rows, us there / here: bf16 4096 x 4096 10.3 / 12.4, 4096 x 11008 21.7 / 21.8, 5120 x 13824
+    (160 tiles on 148 SMs) 34.2 / 29.0; int4 4096 x 8192 17.7 / 14.6, 1536 x 4096 (96 tiles) 9.1 / 8.5.
+    The int8 and int4 lines were drawn before the converting kernel had two groups of converters, and
+    ``uneven`` takes no account of the equal shares that int8 has at three tiles a SM. Against the
+    kernels as they are, over 700 products each of 512 to 32016 features, K of 512 to 22016 and 9 to 16
+    rows, the choice is off the better one by 0.7 % on average for bf16 and int8 and 2.2 % for int4. The
+    farthest off are int4 1024 x 11008 (18.7 there, where it goes, 11.8 here), int8 1024 x 13824 (16.7,
+    13.0), and bf16 2368 x 16384 (17.4, 23.5 here, where it goes)."""
     two = F >= 32 * N_SM * (1 if K >= 2048 else 2)       # tiles per warp: as in csrc/gemm_rows.cu
     tiles = -(-F // (32 if two else 16))
     uneven = -(-tiles // N_SM) * N_SM / tiles if 2 * tiles > N_SM else 1.0
