@@ -213,9 +213,11 @@ umma_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // What bounds the kernel is the conversion: about 12 cycles of a scheduler's ALU per four int8 codes
     // (quant_cvt.cuh). With one group of eight warps its loads, waits and hand-shakes came on top, a gated
     // stage taking 1893 cycles of which 800 without the conversion; two groups overlap them. Chain of
-    // launches, 64 rows, one group and the older conversion -> now, int8 and int4 (us): 12288 x 4096 27.1 -> 21.9
-    // and 27.5 -> 22.9; gated 2 x 11008 x 4096 46.1 -> 37.4 and 48.9 -> 39.6; 4096 x 11008 20.8 -> 17.8 and 21.3
-    // -> 18.5; 4096 x 4096 12.2 -> 11.6. (16 warps on each stage were no faster than eight.)
+    // launches, 64 rows, one group and the older conversion -> two groups, int8 and int4 (us): 12288 x 4096 27.1 ->
+    // 21.9 and 27.5 -> 22.9; gated 2 x 11008 x 4096 46.1 -> 37.4 and 48.9 -> 39.6; 4096 x 11008 20.8 -> 17.8 and
+    // 21.3 -> 18.5; 4096 x 4096 12.2 -> 11.6. (16 warps on each stage were no faster than eight.) With the wait for
+    // the buffer before the one for the stage, timed afresh: 12288 x 4096 22.2 -> 22.0 and 22.9 -> 21.1; gated 33.2
+    // -> 33.3 and 35.4 -> 32.5; 4096 x 11008 18.2 -> 18.0 and 18.3 -> 17.2; 4096 x 4096 11.5 -> 11.4 and 11.4 -> 11.2.
     const bool lead = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, BN, 0, 0);
     // descriptors: constant high word, base low words once, one add per instruction; stage and

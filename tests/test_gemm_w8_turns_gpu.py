@@ -101,3 +101,28 @@ def test_rings(bits, dual, T, ring, trips):
             tol = (K + 2) * 2.0 ** -23 * (x.double().abs() @ f.abs().t()) + 2.0 ** -8 * dual * want.abs()
             assert bool(((out.double() - want).abs() <= 1.01 * tol + 1e-30).all())
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("F,K,T,bits", [(12288, 4096, 128, 8), (15360, 5120, 80, 8), (12288, 4096, 128, 4),
+                                        (2752, 4096, 64, 8), (2752, 8192, 64, 8)])
+def test_odd_rings_as_dispatched(F, K, T, bits):
+    """Shapes whose own ring has an odd number of stages (tests/test_gemm_w8_ring_cpu.py): 5 beside 4 buffers,
+    and gated with K in four (2752 features) 3 beside 3."""
+    from easy_to_hard_b200.ops import _lib, gemm
+    dual = F == 2752
+    g = torch.Generator(device="cuda").manual_seed(F + K)
+    ws = [_weight(F, K, bits, g) for _ in range(1 + dual)]
+    x = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    scale = torch.cat([s for _, s, _ in ws]) if bits == 8 else None
+    outs = [torch.empty(T, F, device="cuda", dtype=torch.bfloat16 if dual else torch.float32) for _ in ws]
+    for _ in range(8):
+        if dual:
+            gemm.gemm(ws[0][0], x, epi=gemm.EPI_DUAL_STORE, a2=ws[1][0], out=outs[0], out2=outs[1], scale=scale)
+        else:
+            gemm.linear(x, ws[0][0], out=outs[0], scale=scale)
+        for out, (_, s, f) in zip(outs, ws):
+            f = f if s is None else f * s.double()[:, None]
+            want = x.double() @ f.t()
+            tol = (K + 2) * 2.0 ** -23 * (x.double().abs() @ f.abs().t()) + 2.0 ** -8 * dual * want.abs()
+            assert bool(((out.double() - want).abs() <= 1.01 * tol + 1e-30).all())
+    assert _lib.read_status() == 0
